@@ -127,7 +127,7 @@ struct sun_ctx {
     DevBuf err;          // device error word (injected-stream overrun)
     size_t hbm_budget = 0;
     // launch shapes (CTA sizes) per kernel family
-    int blk_update = 128, blk_sites = 128, blk_links = 256, blk_wilson = 64;
+    int blk_update = 128, blk_sites = 128, blk_links = 256;
     // update kernel: 0 chosen by size (or by the tuner), 1 always one thread
     // per half-site (k_update), 2 always N lanes per half-site (k_update_rows),
     // 3 the tiled kernel where it applies (k_update_tile: N >= 4, full links).
@@ -211,6 +211,15 @@ int work_of(const LatDev& L, int kind)
     }
 }
 
+int ctas_of(const LatDev& L, int kind, int block)
+{
+    if (kind == WORK_WILSON) {
+        const int per = wilson_per_cta(L.V, block);
+        return (wilson_items(L.V, block) + per - 1) / per;
+    }
+    return (work_of(L, kind) + block - 1) / block;
+}
+
 // Same-class lattices advanced by one launch per kernel.
 struct Group {
     int N = 0, fp64 = 0, layout = 0;
@@ -257,7 +266,7 @@ struct Group {
         if (!e.valid) {
             std::vector<int> b(lats.size() + 1, 0);
             for (size_t i = 0; i < lats.size(); ++i)
-                b[i + 1] = b[i] + (work_of(lats[i]->desc, kind) + block - 1) / block;
+                b[i + 1] = b[i] + ctas_of(lats[i]->desc, kind, block);
             if (!e.buf) e.buf = std::make_shared<DevBuf>();
             e.buf->ensure(sizeof(int) * b.size());
             ck(cudaMemcpyAsync(e.buf->p, b.data(), sizeof(int) * b.size(), cudaMemcpyHostToDevice, s), "begin upload");
@@ -507,6 +516,22 @@ void group_polyakov(sun_ctx* c, Group& g, double* out, cudaStream_t s)
         double norm = (double)g.N * L.X[0] * L.X[1] * L.X[2];
         out[2 * i] = r[2 * i] / norm;
         out[2 * i + 1] = r[2 * i + 1] / norm;
+    }
+}
+
+// 2 (R + 1)(T + 1) doubles per lattice, divided by 3 N V
+void group_wilson(Group& g, int R, int T, cudaStream_t s)
+{
+    BatchView v = g.view(WORK_WILSON, wilson_block(g.N, R, T), s);
+    const size_t nv = 2 * (size_t)(R + 1) * (T + 1);
+    g.partials.ensure(sizeof(double) * 2 * (size_t)std::max(1, wilson_slots(R, T)) * std::max(1, v.nblocks));
+    g.h_out.ensure(sizeof(double) * nv * g.lats.size());
+    double* out = reinterpret_cast<double*>(g.h_out.p);
+    OPS_CALL(g.N, wilson, g.fp64, g.layout, v, R, T, reinterpret_cast<double*>(g.partials.p), out, s);
+    ck(cudaStreamSynchronize(s), "Wilson loops");
+    for (size_t i = 0; i < g.lats.size(); ++i) {
+        const double norm = 3.0 * g.N * (double)g.lats[i]->desc.V;
+        for (size_t k = 0; k < nv; ++k) out[i * nv + k] /= norm;
     }
 }
 
@@ -1374,13 +1399,8 @@ sun_status sun_wilson_loops(sun_lattice* l, int R, int T, double* out, void* str
         if (T >= l->p.dims[3]) fail(SUN_ERR_INVALID_ARG, "T=%d not below temporal extent", T);
         cudaStream_t s = S(l->ctx, stream);
         Solo so(l);
-        const int nv = 2 * (R + 1) * (T + 1);
-        const int blk = l->ctx->blk_wilson;
-        double* r = group_reduce(so.g, WORK_SITES, blk, nv, false, s, [&](const BatchView& v, double* part) {
-            OPS_CALL(l->p.ncolors, wilson, so.g.fp64, so.g.layout, v, blk, R, T, part, s);
-        });
-        const double norm = 3.0 * l->p.ncolors * (double)l->desc.V;
-        for (int i = 0; i < nv; ++i) out[i] = r[i] / norm;
+        group_wilson(so.g, R, T, s);
+        memcpy(out, so.g.h_out.p, sizeof(double) * 2 * (R + 1) * (T + 1));
     });
 }
 
@@ -1803,16 +1823,13 @@ sun_status sun_batch_wilson_loops(sun_batch* b, int R, int T, double* out, void*
         b->regroup();
         cudaStream_t s = S(b->ctx, stream);
         const int nv = 2 * (R + 1) * (T + 1);
-        const int blk = b->ctx->blk_wilson;
         for (auto& g : b->groups) {
             if (g->lats.empty()) continue;
-            double* r = group_reduce(*g, WORK_SITES, blk, nv, false, s, [&](const BatchView& v, double* part) {
-                OPS_CALL(g->N, wilson, g->fp64, g->layout, v, blk, R, T, part, s);
-            });
+            group_wilson(*g, R, T, s);
+            const double* r = reinterpret_cast<const double*>(g->h_out.p);
             for (size_t i = 0; i < g->lats.size(); ++i) {
                 const size_t pos = std::find(b->order.begin(), b->order.end(), g->lats[i]) - b->order.begin();
-                const double norm = 3.0 * g->N * (double)g->lats[i]->desc.V;
-                for (int k = 0; k < nv; ++k) out[pos * nv + k] = r[i * nv + k] / norm;
+                memcpy(out + pos * nv, r + i * nv, sizeof(double) * nv);
             }
         }
     });

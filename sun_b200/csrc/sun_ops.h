@@ -70,8 +70,37 @@ enum UpdateMode { MODE_HB = 0, MODE_HB_INJECTED = 1, MODE_OR = 2 };
 // work items per lattice of a launch: half-sites, sites, spatial sites,
 // links, (site, plane) pairs of the plaquette (6 V), and 8 lanes per spatial
 // site of the Polyakov loop
-enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY8 = 5 };
+enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY8 = 5,
+                WORK_WILSON = 6 };
 constexpr int kPolyLanes = 8;
+// Wilson loops (k_wilson): work items are (tile of `block` consecutive sites,
+// spatial direction), item i = 3 tile + mu, and a CTA takes wilson_per_cta
+// consecutive ones.  kWilsonCtas: the CTAs of one lattice at most -- 3 per SM,
+// what the shared memory of N = 3, T = 4 lets reside, so one lattice's items
+// are spread evenly over one wave.  Both depend on the lattice and the loop
+// extents alone, so the sums have the same bits alone and in a batch.
+constexpr int kWilsonCtas = 444;
+__host__ __device__ inline int wilson_items(int V, int block) { return 3 * ((V + block - 1) / block); }
+__host__ __device__ inline int wilson_per_cta(int V, int block)
+{
+    return (wilson_items(V, block) + kWilsonCtas - 1) / kWilsonCtas;
+}
+// values a launch sums: Re and Im of W(r, t) for r, t > 0, then Re of W(0, t)
+// and of W(r, 0), whose sums are real (W(0, 0) = 1 needs none)
+__host__ __device__ inline int wilson_slots(int R, int T) { return 2 * R * T + T + R; }
+// shared memory of a CTA: the T matrices of each thread and the sums of each warp
+__host__ __device__ inline int wilson_smem(int N, int R, int T, int block)
+{
+    return 16 * (block * T * N * N + block / 32 * wilson_slots(R, T));
+}
+// threads per CTA: the most, up to 128, with which three CTAs fit an SM's
+// 228 KB; 32 where not even 64 do (N >= 4 and large T)
+__host__ __device__ inline int wilson_block(int N, int R, int T)
+{
+    for (int b = 128; b > 32; b -= 32)
+        if (wilson_smem(N, R, T, b) <= 75 * 1024) return b;
+    return 32;
+}
 // lattices below this volume measure the plaquette with one thread per
 // (site, plane), warp-major (a warp: one plane of 32 consecutive sites), the
 // others with one thread per site; the choice depends on the lattice alone
@@ -130,8 +159,8 @@ template <int N> struct Ops {
     // a multiple of reunit_every
     static cudaError_t reunit(int fp64, int layout, const BatchView& bv, int block, int only_due,
                               cudaStream_t s);
-    // per-CTA partials: plaquette 2 values, polyakov 2, wilson 2(R+1)(T+1),
-    // unitarity 1 (max); partial layout [block][value][sum, compensation]
+    // per-CTA partials: plaquette 2 values, polyakov 2, unitarity 1 (max);
+    // partial layout [block][value][sum, compensation]
     // plaquette and polyakov: with out non-null, the last CTA of each
     // lattice also finalizes its sums into out[2 l .. 2 l + 1] (counters: one
     // zeroed unsigned per lattice, left at zero); with slot non-null, into
@@ -147,8 +176,11 @@ template <int N> struct Ops {
     static cudaError_t plaq_poly(int fp64, int layout, const BatchView& vp, const BatchView& vl, double* part_p,
                                  double* part_l, double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
                                  unsigned* slot, unsigned* joint, int end_n_hb, cudaStream_t s);
-    static cudaError_t wilson(int fp64, int layout, const BatchView& bv, int block, int R, int T,
-                              double* partials, cudaStream_t s);
+    // Wilson loops: bv a WORK_WILSON view for wilson_block(N, R, T); partials
+    // hold wilson_slots(R, T) (sum, compensation) pairs per CTA, out
+    // 2 (R + 1)(T + 1) sums per lattice (host-mapped memory allowed)
+    static cudaError_t wilson(int fp64, int layout, const BatchView& bv, int R, int T, double* partials, double* out,
+                              cudaStream_t s);
     static cudaError_t unitarity(int fp64, int layout, const BatchView& bv, int block, double* partials,
                                  cudaStream_t s);
     // sums of tr U and det U over links: 4 values (Re tr, Im tr, Re det, Im det)
