@@ -238,6 +238,14 @@ struct Group {
     bool dirty = true;
     std::vector<unsigned> versions;
 
+    // whether a lattice measures the plaquette with one thread per site
+    int large() const
+    {
+        for (auto* l : lats)
+            if (l->desc.V >= kPlaneSplitMaxV) return 1;
+        return 0;
+    }
+
     void sync(cudaStream_t s)
     {
         if (!dirty) {
@@ -495,7 +503,7 @@ void group_plaquette(sun_ctx* c, Group& g, double* out, cudaStream_t s)
 {
     double* r = group_reduce_fused(g, WORK_PLANES, c->blk_sites, 2, s,
                                    [&](const BatchView& v, double* part, double* out, unsigned* cnt) {
-                                       OPS_CALL(g.N, plaquette, g.fp64, g.layout, v, c->blk_sites, part, out, cnt, nullptr, s);
+                                       OPS_CALL(g.N, plaquette, g.fp64, g.layout, v, g.large(), c->blk_sites, part, out, cnt, nullptr, s);
                                    });
     for (size_t i = 0; i < g.lats.size(); ++i) {
         const LatDev& L = g.lats[i]->desc;
@@ -1167,10 +1175,10 @@ static bool solo_measure_graph(sun_lattice* l, Group& g, int n_hb, int n_or, siz
         group_sweep(c, g, n_hb, n_or, true, re, cs, fused);
         if (fused) {
             unsigned* mc = reinterpret_cast<unsigned*>(l->meas_cnt.p);
-            OPS_CALL(g.N, plaq_poly, g.fp64, g.layout, vp, vl, part, part + 4 * (size_t)vp.nblocks, out_p, out_l, mc,
+            OPS_CALL(g.N, plaq_poly, g.fp64, g.layout, vp, g.large(), vl, part, part + 4 * (size_t)vp.nblocks, out_p, out_l, mc,
                      mc + 1, slot, mc + 2, re ? -1 : n_hb, cs);
         } else {
-            OPS_CALL(g.N, plaquette, g.fp64, g.layout, vp, c->blk_sites, part, out_p, cnt, slot, cs);
+            OPS_CALL(g.N, plaquette, g.fp64, g.layout, vp, g.large(), c->blk_sites, part, out_p, cnt, slot, cs);
             OPS_CALL(g.N, polyakov, g.fp64, g.layout, vl, c->blk_sites, part, out_l, cnt, slot, cs);
             ck(launch_bump(slot, cs), "bump");
         }

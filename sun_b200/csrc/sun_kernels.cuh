@@ -818,35 +818,43 @@ SUN_DEV void block_sum(double v, double* out, DD* sh)
     }
     __syncthreads();
 }
-// Finalize of lattice l's CTA partials, run by the last of its CTAs to
-// finish (each CTA fences its partials, then counts itself in): the same
-// lane-strided compensated sums and shuffle tree as k_finalize_sum, so the
-// result is the same whichever CTA runs it.  The result goes straight to
-// out (host-mapped memory allowed); the counter is left at zero.  slot (may
-// be null): a device counter; the results go to row *slot of out (nlat *
-// nvals doubles per row), so a replayed graph fills one row per replay.
-// The sums of CTA partials b0 .. b1 - 1 (nvals values each), by one warp
-// (lane = threadIdx.x < 32): lane-strided compensated sums, then the shuffle
-// tree; lane 0 writes value v to dst[v].
-SUN_DEV void finalize_partials(const double* partials, int b0, int b1, int nvals, double* dst)
+// The sums of CTA partials b0 .. b1 - 1 (two values each), by a whole CTA:
+// thread-strided compensated sums, the shuffle tree of each warp, then the
+// warps' results in order; thread 0 writes value v to dst[v].  (One warp
+// walking the partials of a 32^4 plaquette, 8,192 CTAs, took 80 us.)
+SUN_DEV void finalize_partials(const double* partials, int b0, int b1, double* dst, DD* sh)
 {
-    const int lane = threadIdx.x;
-    for (int v = 0; v < nvals; ++v) {
-        DD d;
-        d.s = 0.0; d.c = 0.0;
-        for (int b = b0 + lane; b < b1; b += 32) {
-            DD t;
-            t.s = __ldcg(partials + ((size_t)b * nvals + v) * 2);
-            t.c = __ldcg(partials + ((size_t)b * nvals + v) * 2 + 1);
-            d = dd_add(d, t);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    DD d[2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 4
+    for (int b = b0 + (int)threadIdx.x; b < b1; b += (int)blockDim.x)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const double2 p = __ldcg(reinterpret_cast<const double2*>(partials) + 2 * (size_t)b + v);
+            d[v] = dd_add(d[v], DD{p.x, p.y});
         }
-        d = dd_warp(d);
-        if (lane == 0) dst[v] = d.s + d.c;
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        d[v] = dd_warp(d[v]);
+        if (lane == 0) sh[2 * warp + v] = d[v];
     }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        DD t = sh[threadIdx.x];
+        for (int k = 1; k < nw; ++k) t = dd_add(t, sh[2 * k + threadIdx.x]);
+        dst[threadIdx.x] = t.s + t.c;
+    }
+    __syncthreads();
 }
+// Finalize of lattice l's CTA partials (two values each), run by the last of
+// its CTAs to finish (each CTA fences its partials, then counts itself in),
+// so the result is the same whichever CTA runs it.  The result goes straight
+// to out (host-mapped memory allowed); the counter is left at zero.  slot
+// (may be null): a device counter; the results go to row *slot of out (2 nlat
+// doubles per row), so a replayed graph fills one row per replay.
 // Returns (in every thread) whether this CTA was the one that finalized.
-SUN_DEV bool finalize_if_last(const BatchView& bv, int l, const double* partials, int nvals, double* out,
-                              unsigned* counters, const unsigned* slot)
+SUN_DEV bool finalize_if_last(const BatchView& bv, int l, const double* partials, double* out, unsigned* counters,
+                              const unsigned* slot, DD* sh)
 {
     __shared__ int last;
     __threadfence();
@@ -856,13 +864,12 @@ SUN_DEV bool finalize_if_last(const BatchView& bv, int l, const double* partials
         last = atomicAdd(counters + l, 1u) == n - 1u;
     }
     __syncthreads();
-    const bool mine = last != 0;
-    if (!mine || threadIdx.x >= 32) return mine;
+    if (!last) return false;
     __threadfence();
-    const size_t row = slot ? (size_t)__ldcg(slot) * (size_t)bv.nlat * nvals : 0;
-    finalize_partials(partials, __ldg(bv.begin + l), __ldg(bv.begin + l + 1), nvals, out + row + (size_t)l * nvals);
+    const size_t row = slot ? (size_t)__ldcg(slot) * (size_t)bv.nlat * 2 : 0;
+    finalize_partials(partials, __ldg(bv.begin + l), __ldg(bv.begin + l + 1), out + row + (size_t)l * 2, sh);
     if (threadIdx.x == 0) counters[l] = 0u;
-    return mine;
+    return true;
 }
 
 SUN_DEV void block_max(double v, double* out, double* sh)
@@ -933,10 +940,77 @@ SUN_DEV double plaquette_plane(const LatDev& L, const Geom& g, const int x[4], i
     return mtrace_nd(P, Q).re;
 }
 
+// The six planes of one site of a larger lattice (the values of
+// plaquette_plane).  The site's own links U_1 .. U_3(x), used by three planes
+// each, are widened once and kept in shared memory (element e of U_nu at
+// own[((nu - 1) N N + e) stride]), so 16 links are loaded, rebuilt and widened
+// instead of 24 -- the FP32 -> FP64 conversions, not the FP64 products, would
+// bound the kernel otherwise -- and both products and the trace are formed a
+// row at a time.  N = 6 would take 221 KB per CTA and goes plane by plane.
+template <int N> constexpr bool kPlaquetteOwn = N <= 4;
+template <int N> constexpr int plaquette_smem(int block) { return kPlaquetteOwn<N> ? 3 * N * N * 16 * block : 0; }
+template <int N, class R, int LAYOUT>
+SUN_DEV void plaquette_site(const LatDev& L, const Geom& g, const int x[4], double2* own, int stride, double& sp,
+                            double& tp)
+{
+    const int S[4] = {1, g.X[0], g.X[0] * g.X[1], g.X[0] * g.X[1] * g.X[2]};
+    const int lex = lex_of(g, x), par = (x[0] + x[1] + x[2] + x[3]) & 1;
+    const cx<R>* base = reinterpret_cast<const cx<R>*>(L.links);
+    auto load = [&](int at, int p, int mu, Mat<N, double>& A) {
+        Mat<N, R> F;
+        const uint32_t s = L.evenodd ? (uint32_t)((at >> 1) + p * g.halfV) : (uint32_t)at;
+        LinkIO<N, R, LAYOUT>::template load<LD_NC>(base, s + (uint32_t)mu * (uint32_t)g.V, 4u * (uint32_t)g.V, F);
+        mconvert(F, A);
+    };
+    Mat<N, double> A, B, D;
+#pragma unroll 1
+    for (int nu = 1; nu < 4; ++nu) {
+        load(lex, par, nu, B);
+#pragma unroll
+        for (int e = 0; e < N * N; ++e)
+            own[((nu - 1) * N * N + e) * stride] = make_double2(B.e[e / N][e % N].re, B.e[e / N][e % N].im);
+    }
+    load(lex, par, 0, A);
+    sp = 0.0;
+    tp = 0.0;
+#pragma unroll 1
+    for (int mu = 0; mu < 3; ++mu) {
+        if (mu > 0) {
+#pragma unroll
+            for (int e = 0; e < N * N; ++e) {
+                const double2 v = own[((mu - 1) * N * N + e) * stride];
+                A.e[e / N][e % N] = mkc(v.x, v.y);
+            }
+        }
+        const int lm = lex_step(lex, sel4(x, mu), sel4(g.X, mu), sel4(S, mu), 1);
+#pragma unroll 1
+        for (int nu = mu + 1; nu < 4; ++nu) {
+            load(lm, par ^ 1, nu, B);
+            load(lex_step(lex, sel4(x, nu), sel4(g.X, nu), sel4(S, nu), 1), par ^ 1, mu, D);
+            double t = 0.0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                cx<double> c[N], p[N], q[N];
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    const double2 v = own[((nu - 1) * N * N + i * N + j) * stride];
+                    c[j] = mkc(v.x, v.y);
+                }
+                rmul<N, double>(A.e[i], B, p);
+                rmul<N, double>(c, D, q);
+#pragma unroll
+                for (int j = 0; j < N; ++j) t = fma(p[j].im, q[j].im, fma(p[j].re, q[j].re, t));
+            }
+            if (nu == 3) tp += t; else sp += t;
+        }
+    }
+}
+
 // plaquette work item w of lattice L (thread w of k_plaquette's CTAs over
-// the lattice): its spatial and temporal sums, links loaded through path P
+// the lattice): its spatial and temporal sums, links loaded through path P.
+// own: this CTA's shared memory (plaquette_smem), for larger lattices only
 template <int N, class R, int LAYOUT, int P>
-SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, double& tp)
+SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, double& tp, double2* own = nullptr)
 {
     sp = 0.0;
     tp = 0.0;
@@ -954,13 +1028,17 @@ SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, d
     } else if (w < g.V) {
         int x[4];
         lex_coords(g, w, x);
+        if constexpr (kPlaquetteOwn<N> && P == LD_NC) {
+            plaquette_site<N, R, LAYOUT>(L, g, x, own + threadIdx.x, blockDim.x, sp, tp);
+        } else {
 #pragma unroll 1
-        for (int mu = 0; mu < 3; ++mu)
+            for (int mu = 0; mu < 3; ++mu)
 #pragma unroll 1
-            for (int nu = mu + 1; nu < 4; ++nu) {
-                const double t = plaquette_plane<N, R, LAYOUT, P>(L, g, x, mu, nu);
-                if (nu == 3) tp += t; else sp += t;
-            }
+                for (int nu = mu + 1; nu < 4; ++nu) {
+                    const double t = plaquette_plane<N, R, LAYOUT, P>(L, g, x, mu, nu);
+                    if (nu == 3) tp += t; else sp += t;
+                }
+        }
     }
 }
 
@@ -968,6 +1046,7 @@ template <int N, class R, int LAYOUT>
 __global__ void __launch_bounds__(128) k_plaquette(BatchView bv, double* partials, double* out, unsigned* counters,
                                                     const unsigned* slot)
 {
+    extern __shared__ __align__(16) unsigned char plaquette_raw[];
     __shared__ DD sh[32];
     const int b = blockIdx.x;
     const int l = find_lat(bv, b);
@@ -975,10 +1054,10 @@ __global__ void __launch_bounds__(128) k_plaquette(BatchView bv, double* partial
     const Geom g = geom_of(L);
     const int w = (b - __ldg(bv.begin + l)) * blockDim.x + threadIdx.x;
     double sp, tp;
-    plaquette_item<N, R, LAYOUT, LD_NC>(L, g, w, sp, tp);
+    plaquette_item<N, R, LAYOUT, LD_NC>(L, g, w, sp, tp, reinterpret_cast<double2*>(plaquette_raw));
     block_sum(sp, partials + (size_t)b * 4, sh);
     block_sum(tp, partials + (size_t)b * 4 + 2, sh);
-    if (out) finalize_if_last(bv, l, partials, 2, out, counters, slot);
+    if (out) finalize_if_last(bv, l, partials, out, counters, slot, sh);
 }
 
 template <int N> SUN_DEV void shfl_mat(Mat<N, double>& D, const Mat<N, double>& S, int src)
@@ -1056,7 +1135,7 @@ __global__ void __launch_bounds__(128) k_polyakov(BatchView bv, double* partials
     polyakov_item<N, R, LAYOUT, LD_NC>(L, g, w, re, im);
     block_sum(re, partials + (size_t)b * 4, sh);
     block_sum(im, partials + (size_t)b * 4 + 2, sh);
-    if (out) finalize_if_last(bv, l, partials, 2, out, counters, slot);
+    if (out) finalize_if_last(bv, l, partials, out, counters, slot, sh);
 }
 
 // The plaquette and the Polyakov loop in one launch (the measurements of a
@@ -1071,6 +1150,7 @@ __global__ void __launch_bounds__(128) k_plaq_poly(BatchView vp, BatchView vl, d
                                                     double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
                                                     unsigned* slot, unsigned* joint, int end_n_hb)
 {
+    extern __shared__ __align__(16) unsigned char plaquette_raw[];
     __shared__ DD sh[32];
     const bool plaq = (int)blockIdx.x < vp.nblocks;
     const BatchView& bv = plaq ? vp : vl;
@@ -1080,12 +1160,12 @@ __global__ void __launch_bounds__(128) k_plaq_poly(BatchView vp, BatchView vl, d
     const Geom g = geom_of(L);
     const int w = (b - __ldg(bv.begin + l)) * blockDim.x + threadIdx.x;
     double v0, v1;
-    if (plaq) plaquette_item<N, R, LAYOUT, LD_NC>(L, g, w, v0, v1);
+    if (plaq) plaquette_item<N, R, LAYOUT, LD_NC>(L, g, w, v0, v1, reinterpret_cast<double2*>(plaquette_raw));
     else polyakov_item<N, R, LAYOUT, LD_NC>(L, g, w, v0, v1);
     double* part = plaq ? part_p : part_l;
     block_sum(v0, part + (size_t)b * 4, sh);
     block_sum(v1, part + (size_t)b * 4 + 2, sh);
-    const bool fin = finalize_if_last(bv, l, part, 2, plaq ? out_p : out_l, plaq ? cnt_p : cnt_l, slot);
+    const bool fin = finalize_if_last(bv, l, part, plaq ? out_p : out_l, plaq ? cnt_p : cnt_l, slot, sh);
     if (fin && threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(joint, 1u) == 2u * (unsigned)vp.nlat - 1u) {
@@ -1679,8 +1759,8 @@ __global__ void __launch_bounds__(128) k_sweeps_resident(ResidentArgs a)
         // finalized by two CTAs of set 1, which starts the next sweep second;
         // the partials are written again only after the next sweep's
         // barriers, which these CTAs reach after their finalize
-        if (blockIdx.x == P && threadIdx.x < 32) finalize_partials(a.partials, 0, a.plaq.nblocks, 2, a.out_plaq + 2 * sw);
-        if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 32) finalize_partials(ppart, 0, a.poly.nblocks, 2, a.out_poly + 2 * sw);
+        if (blockIdx.x == P) finalize_partials(a.partials, 0, a.plaq.nblocks, a.out_plaq + 2 * sw, sh);
+        if (blockIdx.x == gridDim.x - 1) finalize_partials(ppart, 0, a.poly.nblocks, a.out_poly + 2 * sw, sh);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         L.state[0] += (unsigned)(a.n_sweeps * a.n_hb);
@@ -1859,14 +1939,27 @@ cudaError_t Ops<N>::reunit(int fp64, int layout, const BatchView& bv, int block,
     return cudaGetLastError();
 }
 
+// the shared memory of a large lattice's plaquette (above 48 KB for N >= 3),
+// opted in once per instance
+template <int N, auto KERNEL> cudaError_t allow_plaquette_smem()
+{
+    static const cudaError_t e =
+        cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, plaquette_smem<N>(128));
+    return e;
+}
+
 template <int N>
-cudaError_t Ops<N>::plaquette(int fp64, int layout, const BatchView& bv, int block, double* partials,
+cudaError_t Ops<N>::plaquette(int fp64, int layout, const BatchView& bv, int large, int block, double* partials,
                               double* out, unsigned* counters, const unsigned* slot, cudaStream_t s)
 {
-#define CALL(R_, L_) k_plaquette<N, R_, L_><<<bv.nblocks, block, 0, s>>>(bv, partials, out, counters, slot)
+    const int smem = large ? plaquette_smem<N>(block) : 0;
+    cudaError_t e = cudaSuccess;
+#define CALL(R_, L_)                                                                                        \
+    if ((e = allow_plaquette_smem<N, k_plaquette<N, R_, L_>>()) == cudaSuccess)                               \
+        k_plaquette<N, R_, L_><<<bv.nblocks, block, smem, s>>>(bv, partials, out, counters, slot)
     SUN_DISPATCH(fp64, layout, CALL);
 #undef CALL
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <int N>
@@ -1880,16 +1973,19 @@ cudaError_t Ops<N>::polyakov(int fp64, int layout, const BatchView& bv, int bloc
 }
 
 template <int N>
-cudaError_t Ops<N>::plaq_poly(int fp64, int layout, const BatchView& vp, const BatchView& vl, double* part_p,
+cudaError_t Ops<N>::plaq_poly(int fp64, int layout, const BatchView& vp, int large, const BatchView& vl, double* part_p,
                               double* part_l, double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
                               unsigned* slot, unsigned* joint, int end_n_hb, cudaStream_t s)
 {
-#define CALL(R_, L_)                                                                                          \
-    k_plaq_poly<N, R_, L_><<<vp.nblocks + vl.nblocks, 128, 0, s>>>(vp, vl, part_p, part_l, out_p, out_l, cnt_p, \
-                                                                    cnt_l, slot, joint, end_n_hb)
+    const int smem = large ? plaquette_smem<N>(128) : 0;
+    cudaError_t e = cudaSuccess;
+#define CALL(R_, L_)                                                                                            \
+    if ((e = allow_plaquette_smem<N, k_plaq_poly<N, R_, L_>>()) == cudaSuccess)                                   \
+        k_plaq_poly<N, R_, L_><<<vp.nblocks + vl.nblocks, 128, smem, s>>>(vp, vl, part_p, part_l, out_p, out_l, \
+                                                                          cnt_p, cnt_l, slot, joint, end_n_hb)
     SUN_DISPATCH(fp64, layout, CALL);
 #undef CALL
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // the instance's shared memory is opted in once, at the most any R, T <= 8 takes

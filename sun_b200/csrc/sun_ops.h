@@ -165,7 +165,8 @@ template <int N> struct Ops {
     // lattice also finalizes its sums into out[2 l .. 2 l + 1] (counters: one
     // zeroed unsigned per lattice, left at zero); with slot non-null, into
     // row *slot of out (2 nlat doubles per row)
-    static cudaError_t plaquette(int fp64, int layout, const BatchView& bv, int block, double* partials,
+    // large: a lattice of the view has at least kPlaneSplitMaxV sites
+    static cudaError_t plaquette(int fp64, int layout, const BatchView& bv, int large, int block, double* partials,
                                  double* out, unsigned* counters, const unsigned* slot, cudaStream_t s);
     static cudaError_t polyakov(int fp64, int layout, const BatchView& bv, int block, double* partials,
                                 double* out, unsigned* counters, const unsigned* slot, cudaStream_t s);
@@ -173,8 +174,8 @@ template <int N> struct Ops {
     // for 128), the last finalize advancing *slot
     // end_n_hb >= 0: the same launch ends the sweep (advance_counters with
     // n_hb = end_n_hb, one sweep) after the measurements
-    static cudaError_t plaq_poly(int fp64, int layout, const BatchView& vp, const BatchView& vl, double* part_p,
-                                 double* part_l, double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
+    static cudaError_t plaq_poly(int fp64, int layout, const BatchView& vp, int large, const BatchView& vl,
+                                 double* part_p, double* part_l, double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
                                  unsigned* slot, unsigned* joint, int end_n_hb, cudaStream_t s);
     // Wilson loops: bv a WORK_WILSON view for wilson_block(N, R, T); partials
     // hold wilson_slots(R, T) (sum, compensation) pairs per CTA, out
