@@ -58,6 +58,9 @@ void ck(cudaError_t e, const char* what)
 // before every further device allocation reports out-of-memory; -1 = off.
 std::atomic<int> g_alloc_budget{-1};
 
+// frees scratch that contexts keep between calls; whether there was any
+bool release_kept_scratch();
+
 // Device buffer owned by the library.
 struct DevBuf {
     void* p = nullptr;
@@ -80,7 +83,13 @@ struct DevBuf {
         while (left > 0 && !g_alloc_budget.compare_exchange_weak(left, left - 1)) {
         }
         if (left == 0) fail(SUN_ERR_OUT_OF_MEMORY, "cudaMalloc: out of memory (injected)");
-        ck(cudaMalloc(&p, bytes), "cudaMalloc");
+        cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (release_kept_scratch()) e = cudaMalloc(&p, bytes);
+        }
+        if (e != cudaSuccess) p = nullptr;
+        ck(e, "cudaMalloc");
         n = bytes;
     }
 };
@@ -157,6 +166,9 @@ struct sun_ctx {
     int skip_arrive = -1;  // test hook (sun_debug_resident_barrier)
     DevBuf res_sync;       // barrier count, generation, status
     DevBuf res_out;        // per-sweep plaquette and Polyakov sums
+    // scratch images kept between calls (ScratchLease), freed with the context
+    // or when an allocation fails
+    std::vector<std::unique_ptr<DevBuf>> kept;
     // autotuner (tuneLaunch, src/tune.cpp:304): CTA size of the update kernel
     // per (kernel class, total half-volume), timed once, cached in a CSV file
     bool tune = false;
@@ -196,6 +208,73 @@ struct sun_lattice {
 };
 
 namespace {
+
+// every live context, for release_kept_scratch
+std::mutex g_ctxs_mu;
+std::vector<sun_ctx*> g_ctxs;
+
+bool release_kept_scratch()
+{
+    bool any = false;
+    std::lock_guard<std::mutex> lk(g_ctxs_mu);
+    for (sun_ctx* c : g_ctxs)
+        if (c->mu.try_lock()) {  // another thread's context in a call keeps its scratch
+            any |= !c->kept.empty();
+            c->kept.clear();
+            c->mu.unlock();
+        }
+    return any;
+}
+
+// Scratch images of one call (a smearing step's second image, HYP levels, the
+// canonical copy of a conversion).  A cudaMalloc and cudaFree of these sizes
+// cost more than the work on them (SU(3) 24^4: APE in FP64 1 ms of 3 ms, HYP in
+// FP32 2.5 ms of 4.7 ms per call), so up to kScratchKeep bytes stay with the
+// context for the next call.  Calls that lease scratch hold the context's lock
+// and synchronise their stream before they return, so no two ever use a buffer
+// at once, whatever their streams; a call that throws synchronises here.
+constexpr size_t kScratchKeep = (size_t)2 << 30;
+class ScratchLease {
+    sun_ctx* c;
+    cudaStream_t s;
+    int exceptions = std::uncaught_exceptions();
+    std::vector<std::unique_ptr<DevBuf>> bufs;
+
+public:
+    ScratchLease(sun_ctx* c_, cudaStream_t s_) : c(c_), s(s_) {}
+    ScratchLease(const ScratchLease&) = delete;
+    void* get(size_t bytes)
+    {
+        auto best = c->kept.end();
+        for (auto it = c->kept.begin(); it != c->kept.end(); ++it)
+            if ((*it)->n >= bytes && (best == c->kept.end() || (*it)->n < (*best)->n)) best = it;
+        if (best != c->kept.end()) {
+            bufs.push_back(std::move(*best));
+            c->kept.erase(best);
+        } else {
+            auto b = std::make_unique<DevBuf>();
+            b->ensure(bytes);
+            bufs.push_back(std::move(b));
+        }
+        return bufs.back()->p;
+    }
+    ~ScratchLease()
+    {
+        if (std::uncaught_exceptions() > exceptions) cudaStreamSynchronize(s);
+        size_t total = 0;
+        for (auto& b : c->kept) total += b->n;
+        for (auto& b : bufs) {
+            // the buffers just used stay, older ones make room
+            while (!c->kept.empty() && total + b->n > kScratchKeep) {
+                total -= c->kept.front()->n;
+                c->kept.erase(c->kept.begin());
+            }
+            if (total + b->n > kScratchKeep) continue;
+            total += b->n;
+            c->kept.push_back(std::move(b));
+        }
+    }
+};
 
 cudaStream_t S(sun_ctx* c, void* s) { return s ? reinterpret_cast<cudaStream_t>(s) : c->stream; }
 
@@ -806,6 +885,10 @@ sun_status sun_init(const sun_config* cfg, sun_ctx** out)
         if (const char* t = getenv("SUN_B200_RESIDENT")) c->resident = !strcmp(t, "auto") ? -1 : (atoi(t) ? 1 : 0);
         if (const char* t = getenv("SUN_B200_RESIDENT_MAX_HALFV")) c->resident_max_halfv = atoll(t);
         if (const char* t = getenv("SUN_B200_PDL")) c->pdl = atoi(t) ? 1 : 0;
+        {
+            std::lock_guard<std::mutex> lk(g_ctxs_mu);
+            g_ctxs.push_back(c.get());
+        }
         *out = c.release();
     });
 }
@@ -813,6 +896,10 @@ sun_status sun_init(const sun_config* cfg, sun_ctx** out)
 sun_status sun_finalize(sun_ctx* c)
 {
     if (!c) return SUN_ERR_INVALID_ARG;
+    {
+        std::lock_guard<std::mutex> lk(g_ctxs_mu);
+        g_ctxs.erase(std::remove(g_ctxs.begin(), g_ctxs.end(), c), g_ctxs.end());
+    }
     cudaStreamSynchronize(c->stream);
     cudaStreamDestroy(c->stream);
     delete c;
@@ -902,12 +989,12 @@ static void canon_upload(sun_lattice* l, const void* host, cudaStream_t s, bool 
 {
     const size_t V = l->desc.V, N = l->p.ncolors;
     const size_t bytes = V * 4 * N * N * 16;
-    DevBuf stage;
+    ScratchLease scratch(l->ctx, s);
     const void* src = host;
     if (!host_is_device) {
-        stage.ensure(bytes);
-        ck(cudaMemcpyAsync(stage.p, host, bytes, cudaMemcpyHostToDevice, s), "upload");
-        src = stage.p;
+        void* stage = scratch.get(bytes);
+        ck(cudaMemcpyAsync(stage, host, bytes, cudaMemcpyHostToDevice, s), "upload");
+        src = stage;
     }
     Solo so(l);
     BatchView v = so.g.view(WORK_LINKS, l->ctx->blk_links, s);
@@ -919,12 +1006,12 @@ static void canon_download(sun_lattice* l, void* host, cudaStream_t s)
 {
     const size_t V = l->desc.V, N = l->p.ncolors;
     const size_t bytes = V * 4 * N * N * 16;
-    DevBuf stage;
-    stage.ensure(bytes);
+    ScratchLease scratch(l->ctx, s);
+    void* stage = scratch.get(bytes);
     Solo so(l);
     BatchView v = so.g.view(WORK_LINKS, l->ctx->blk_links, s);
-    OPS_CALL(l->p.ncolors, unpack, so.g.fp64, so.g.layout, v, l->ctx->blk_links, stage.p, s);
-    ck(cudaMemcpyAsync(host, stage.p, bytes, cudaMemcpyDeviceToHost, s), "download");
+    OPS_CALL(l->p.ncolors, unpack, so.g.fp64, so.g.layout, v, l->ctx->blk_links, stage, s);
+    ck(cudaMemcpyAsync(host, stage, bytes, cudaMemcpyDeviceToHost, s), "download");
     ck(cudaStreamSynchronize(s), "download");
 }
 
@@ -979,25 +1066,29 @@ sun_status sun_lattice_download_async(sun_lattice* l, void* host_image, void* st
 extern "C++" {
 namespace {
 
-// dst <- src through the canonical FP64 order (layout, order and precision
-// conversion); the RNG counters travel with the links
+// dst <- src; the RNG counters travel with the links.  Lattices of one class
+// and order hold the same image, which is copied as it is; otherwise through
+// the canonical FP64 order (layout, order and precision conversion).
 void copy_links(sun_lattice* dst, sun_lattice* src, cudaStream_t s)
 {
     if (dst->p.ncolors != src->p.ncolors) fail(SUN_ERR_INVALID_ARG, "copy between different N");
     for (int k = 0; k < 4; ++k)
         if (dst->p.dims[k] != src->p.dims[k]) fail(SUN_ERR_INVALID_ARG, "copy between different geometries");
     const size_t V = src->desc.V, N = src->p.ncolors;
-    DevBuf stage;
-    stage.ensure(V * 4 * N * N * 16);
-    {
-        Solo so(src);
-        BatchView v = so.g.view(WORK_LINKS, src->ctx->blk_links, s);
-        OPS_CALL(src->p.ncolors, unpack, so.g.fp64, so.g.layout, v, src->ctx->blk_links, stage.p, s);
-    }
-    {
+    ScratchLease scratch(dst->ctx, s);
+    if (dst->p.layout == src->p.layout && dst->p.order == src->p.order && dst->p.precision == src->p.precision) {
+        if (dst != src)
+            ck(cudaMemcpyAsync(dst->links.p, src->links.p, src->bytes, cudaMemcpyDeviceToDevice, s), "copy");
+    } else {
+        void* stage = scratch.get(V * 4 * N * N * 16);
+        {
+            Solo so(src);
+            BatchView v = so.g.view(WORK_LINKS, src->ctx->blk_links, s);
+            OPS_CALL(src->p.ncolors, unpack, so.g.fp64, so.g.layout, v, src->ctx->blk_links, stage, s);
+        }
         Solo so(dst);
         BatchView v = so.g.view(WORK_LINKS, dst->ctx->blk_links, s);
-        OPS_CALL(dst->p.ncolors, pack, so.g.fp64, so.g.layout, v, dst->ctx->blk_links, stage.p, s);
+        OPS_CALL(dst->p.ncolors, pack, so.g.fp64, so.g.layout, v, dst->ctx->blk_links, stage, s);
     }
     ck(cudaMemcpyAsync(dst->state.p, src->state.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToDevice, s), "copy");
     ck(cudaStreamSynchronize(s), "copy");
@@ -1415,8 +1506,10 @@ sun_status sun_wilson_loops(sun_lattice* l, int R, int T, double* out, void* str
 // ---------------------------------------------------------------------------
 // Smearing (src/smear/*.cu).  Each step rebuilds the selected directions from
 // the unchanged field: the steps alternate between the lattice's image and a
-// scratch copy (the unselected directions are equal in both), and an odd
-// step count ends with one copy back.
+// scratch image that only ever holds the selected directions (the others are
+// read from the lattice's image, which keeps them).  The last step has to write
+// the lattice's image, so an odd step count begins with a copy of the selected
+// directions.
 extern "C++" {
 namespace {
 
@@ -1427,17 +1520,30 @@ void check_dirmask(int dirmask)
     if (dirmask <= 0 || dirmask > 15) fail(SUN_ERR_INVALID_ARG, "direction mask %d not in 1..15", dirmask);
 }
 
-template <class F> void smear_steps(sun_lattice* l, int steps, cudaStream_t s, F step)
+// the links of the directions in dirmask, from one image of l to another
+void copy_directions(sun_lattice* l, void* dst, const void* src, int dirmask, cudaStream_t s)
+{
+    const size_t csz = l->p.precision == SUN_F64 ? 16 : 8, row = csz * (size_t)l->desc.V;  // one direction of one element
+    for (int mu = 0; mu < 4;) {
+        int n = 0;
+        while (mu + n < 4 && ((dirmask >> (mu + n)) & 1)) ++n;
+        if (n)
+            ck(cudaMemcpy2DAsync((char*)dst + mu * row, 4 * row, (const char*)src + mu * row, 4 * row, n * row,
+                                 elems_of(l->p.ncolors, l->p.layout), cudaMemcpyDeviceToDevice, s),
+               "smear scratch");
+        mu += n + 1;
+    }
+}
+
+// step(group, view, image of the selected directions, image to write)
+template <class F> void smear_steps(sun_lattice* l, int steps, int dirmask, ScratchLease& scratch, cudaStream_t s, F step)
 {
     if (steps <= 0) return;
-    DevBuf tmp;
-    tmp.ensure(l->bytes);
-    ck(cudaMemcpyAsync(tmp.p, l->links.p, l->bytes, cudaMemcpyDeviceToDevice, s), "smear scratch");
+    void* img[2] = {scratch.get(l->bytes), l->links.p};
     Solo so(l);
     BatchView v = so.g.view(WORK_SITES, kSmearBlock, s);
-    void* img[2] = {l->links.p, tmp.p};
-    for (int st = 0; st < steps; ++st) step(so.g, v, img[st & 1], img[(st + 1) & 1]);
-    if (steps & 1) ck(cudaMemcpyAsync(l->links.p, tmp.p, l->bytes, cudaMemcpyDeviceToDevice, s), "smear copy");
+    if (steps & 1) copy_directions(l, img[0], img[1], dirmask, s);
+    for (int st = steps; st > 0; --st) step(so.g, v, img[(st + 1) & 1], img[st & 1]);
     ck(cudaStreamSynchronize(s), "smearing");
 }
 
@@ -1460,7 +1566,8 @@ sun_status sun_smear_ape(sun_lattice* l, double w, int steps, int nhits, double 
     return handle(l->ctx, [&] {
         check_dirmask(dirmask);
         cudaStream_t s = S(l->ctx, stream);
-        smear_steps(l, steps, s, [&](Group& g, const BatchView& v, const void* src, void* dst) {
+        ScratchLease scratch(l->ctx, s);
+        smear_steps(l, steps, dirmask, scratch, s, [&](Group& g, const BatchView& v, const void* src, void* dst) {
             OPS_CALL(g.N, ape, g.fp64, g.layout, v, kSmearBlock, src, dst, dirmask, w, nhits, tol, s);
         });
     });
@@ -1473,7 +1580,8 @@ sun_status sun_smear_stout(sun_lattice* l, double w, int steps, int dirmask, voi
         check_dirmask(dirmask);
         if (l->p.ncolors != 3) fail(SUN_ERR_UNSUPPORTED, "stout smearing is defined for SU(3) only");
         cudaStream_t s = S(l->ctx, stream);
-        smear_steps(l, steps, s, [&](Group& g, const BatchView& v, const void* src, void* dst) {
+        ScratchLease scratch(l->ctx, s);
+        smear_steps(l, steps, dirmask, scratch, s, [&](Group& g, const BatchView& v, const void* src, void* dst) {
             OPS_CALL(g.N, stout, g.fp64, g.layout, v, kSmearBlock, src, dst, dirmask, w, s);
         });
     });
@@ -1490,13 +1598,12 @@ sun_status sun_smear_hyp(sun_lattice* l, const double alpha[3], int steps, int n
         const double a1 = (float)alpha[0], a2 = (float)alpha[1], a3 = (float)alpha[2];
         const size_t nn = (size_t)l->p.ncolors * l->p.ncolors;
         const size_t slot_bytes = nn * (size_t)l->desc.V * (l->p.precision == SUN_F64 ? 16 : 8);
-        DevBuf b1, b2;
-        b1.ensure(16 * slot_bytes);
-        b2.ensure(16 * slot_bytes);
-        smear_steps(l, steps, s, [&](Group& g, const BatchView& v, const void* src, void* dst) {
-            OPS_CALL(g.N, hyp, g.fp64, g.layout, v, kSmearBlock, 1, src, b1.p, b2.p, dst, dirmask, a3, nhits, tol, s);
-            OPS_CALL(g.N, hyp, g.fp64, g.layout, v, kSmearBlock, 2, src, b1.p, b2.p, dst, dirmask, a2, nhits, tol, s);
-            OPS_CALL(g.N, hyp, g.fp64, g.layout, v, kSmearBlock, 3, src, b1.p, b2.p, dst, dirmask, a1, nhits, tol, s);
+        ScratchLease scratch(l->ctx, s);
+        void *b1 = scratch.get(16 * slot_bytes), *b2 = scratch.get(16 * slot_bytes);
+        smear_steps(l, steps, dirmask, scratch, s, [&](Group& g, const BatchView& v, const void* src, void* dst) {
+            OPS_CALL(g.N, hyp, g.fp64, g.layout, v, kSmearBlock, 1, src, b1, b2, dst, dirmask, a3, nhits, tol, s);
+            OPS_CALL(g.N, hyp, g.fp64, g.layout, v, kSmearBlock, 2, src, b1, b2, dst, dirmask, a2, nhits, tol, s);
+            OPS_CALL(g.N, hyp, g.fp64, g.layout, v, kSmearBlock, 3, src, b1, b2, dst, dirmask, a1, nhits, tol, s);
         });
     });
 }

@@ -193,7 +193,8 @@ template <int N> struct Ops {
     static cudaError_t unpack(int fp64, int layout, const BatchView& bv, int block, void* canon,
                               cudaStream_t s);
     // smearing: src and dst are distinct device images of the lattice, the
-    // launch rows are the directions in dirmask (bit mu selects mu)
+    // launch rows are the directions in dirmask (bit mu selects mu), read from
+    // src; the other directions are read from the lattice's own image
     static cudaError_t ape(int fp64, int layout, const BatchView& bv, int block, const void* src, void* dst,
                            int dirmask, double w, int nhits, double tol, cudaStream_t s);
     static cudaError_t stout(int fp64, int layout, const BatchView& bv, int block, const void* src, void* dst,

@@ -2,9 +2,10 @@
 // hyp.cu, multihit.cu, multihitsp.cu) and their Ops<N> launch wrappers.
 // Included at the end of sun_kernels.cuh.
 //
-// Every kernel reads the unchanged field `src` and writes `dst` (distinct
-// device images of one lattice's layout, order and precision), one thread per
-// site and one grid row (blockIdx.y) per smeared direction or intermediate
+// Every kernel of a smearing step reads the unchanged field and writes `dst`:
+// the smeared directions (dirmask) from `src`, the others from the lattice's
+// own image (src and dst are distinct images of its layout, order and
+// precision; one of them may be that image), one thread per site and one grid row (blockIdx.y) per smeared direction or intermediate
 // link, so a smearing step is one launch (three for HYP) whatever the
 // directions.  The reference allows only normal-order SOA arrays here
 // (src/smear/ape.cu:194-197); these kernels take any storage order and layout.
@@ -23,6 +24,12 @@ SUN_DEV int nth_dir(int dirmask, int row)
             --row;
         }
     return mu;
+}
+
+// the image that holds direction mu of the field a step reads
+SUN_DEV const void* field_of(const LatDev& L, const void* src, int dirmask, int mu)
+{
+    return (dirmask >> mu) & 1 ? src : L.links;
 }
 
 // link (x, mu) of a device image
@@ -62,16 +69,19 @@ SUN_DEV void plane_staple(const Geom& g, const int x[4], int a, int r, GR get_r,
 
 // staple of the link (x, mu) over the planes nu in numask (nu != mu), nu
 // ascending -- kernel_APE_Space (src/smear/ape.cu:44) with numask = 7
+// of the field (src, dirmask)
 template <int N, class R, int LAYOUT>
-SUN_DEV void staple_planes(const LatDev& L, const Geom& g, const void* img, const int x[4], int mu, int numask,
-                           Mat<N, R>& S)
+SUN_DEV void staple_planes(const LatDev& L, const Geom& g, const void* src, int dirmask, const int x[4], int mu,
+                           int numask, Mat<N, R>& S)
 {
     mzero(S);
+    const void* img = field_of(L, src, dirmask, mu);
     auto get_mu = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, img, y, mu, M); };
 #pragma unroll 1
     for (int nu = 0; nu < 4; ++nu) {
         if (nu == mu || !((numask >> nu) & 1)) continue;
-        auto get_nu = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, img, y, nu, M); };
+        const void* other = field_of(L, src, dirmask, nu);
+        auto get_nu = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, other, y, nu, M); };
         plane_staple<N, R>(g, x, mu, nu, get_nu, get_mu, S);
     }
 }
@@ -203,7 +213,7 @@ __global__ void __launch_bounds__(128) k_ape(BatchView bv, const void* src, void
     int x[4];
     site_coords(L, g, site, x);
     Mat<N, R> S, U, W;
-    staple_planes<N, R, LAYOUT>(L, g, src, x, mu, 7, S);
+    staple_planes<N, R, LAYOUT>(L, g, src, dirmask, x, mu, 7, S);
     ld_site<N, R, LAYOUT>(L, g, src, x, mu, U);
     const R inv = R(1) / (R(1) + R(6) * w);
 #pragma unroll
@@ -240,7 +250,7 @@ __global__ void __launch_bounds__(128) k_stout(BatchView bv, const void* src, vo
     int x[4];
     site_coords(L, g, site, x);
     Mat<3, R> S, U, Om, Q, E;
-    staple_planes<3, R, LAYOUT>(L, g, src, x, mu, 7, S);
+    staple_planes<3, R, LAYOUT>(L, g, src, dirmask, x, mu, 7, S);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -287,7 +297,8 @@ SUN_DEV void st_slot(const Geom& g, void* B, int site, int slot, const Mat<N, R>
 // level 1: Vbar_{m;e}(x) = P[(1 - a3) U_m(x) + a3/2 staple of U_m in plane (m, e)]
 // (HYPSmearVbar, hyp.cu:88); grid row = m * 3 + (index of e among e != m)
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128) k_hyp1(BatchView bv, const void* src, void* B1, R a3, int nhits, R tol)
+__global__ void __launch_bounds__(128) k_hyp1(BatchView bv, const void* src, void* B1, int dirmask, R a3, int nhits,
+                                              R tol)
 {
     const int b = blockIdx.x;
     const int l = find_lat(bv, b);
@@ -300,10 +311,11 @@ __global__ void __launch_bounds__(128) k_hyp1(BatchView bv, const void* src, voi
     site_coords(L, g, site, x);
     Mat<N, R> S, U;
     mzero(S);
-    auto get_e = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, src, y, e, M); };
-    auto get_m = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, src, y, m, M); };
+    const void *img_e = field_of(L, src, dirmask, e), *img_m = field_of(L, src, dirmask, m);
+    auto get_e = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, img_e, y, e, M); };
+    auto get_m = [&](const int* y, Mat<N, R>& M) { ld_site<N, R, LAYOUT>(L, g, img_m, y, m, M); };
     plane_staple<N, R>(g, x, m, e, get_e, get_m, S);
-    ld_site<N, R, LAYOUT>(L, g, src, x, m, U);
+    ld_site<N, R, LAYOUT>(L, g, img_m, x, m, U);
     const R h = R(0.5) * a3, c = R(1) - a3;
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -320,8 +332,8 @@ __global__ void __launch_bounds__(128) k_hyp1(BatchView bv, const void* src, voi
 // Vbar_{a;s} with Vbar_{r;s}, s the fourth direction] (HYPSmearVtil,
 // hyp.cu:106); grid row = a * 3 + (index of b among b != a)
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128) k_hyp2(BatchView bv, const void* src, const void* B1, void* B2, R a2,
-                                              int nhits, R tol)
+__global__ void __launch_bounds__(128) k_hyp2(BatchView bv, const void* src, const void* B1, void* B2, int dirmask,
+                                              R a2, int nhits, R tol)
 {
     const int b = blockIdx.x;
     const int l = find_lat(bv, b);
@@ -342,7 +354,7 @@ __global__ void __launch_bounds__(128) k_hyp2(BatchView bv, const void* src, con
         auto get_a = [&](const int* y, Mat<N, R>& M) { ld_slot<N, R>(g, B1, site_index(L, g, y), a * 4 + s, M); };
         plane_staple<N, R>(g, x, a, r, get_r, get_a, S);
     }
-    ld_site<N, R, LAYOUT>(L, g, src, x, a, U);
+    ld_site<N, R, LAYOUT>(L, g, field_of(L, src, dirmask, a), x, a, U);
     const R h = R(0.25) * a2, c = R(1) - a2;
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -412,7 +424,7 @@ __global__ void __launch_bounds__(128) k_multihit(BatchView bv, const void* src,
     int x[4];
     site_coords(L, g, site, x);
     Mat<N, R> S, U, A;
-    staple_planes<N, R, LAYOUT>(L, g, src, x, 3, 15, S);
+    staple_planes<N, R, LAYOUT>(L, g, src, 15, x, 3, 15, S);
     ld_site<N, R, LAYOUT>(L, g, src, x, 3, U);
     A = U;
     PhiloxStream<R> st;
@@ -452,7 +464,7 @@ __global__ void __launch_bounds__(128) k_multihit_space(BatchView bv, const void
     int x[4];
     site_coords(L, g, site, x);
     Mat<N, R> S, U, A;
-    staple_planes<N, R, LAYOUT>(L, g, src, x, m, 7, S);
+    staple_planes<N, R, LAYOUT>(L, g, src, 15, x, m, 7, S);
     ld_site<N, R, LAYOUT>(L, g, src, x, m, U);
     mzero(A);
 #pragma unroll 1
@@ -508,8 +520,8 @@ cudaError_t Ops<N>::hyp(int fp64, int layout, const BatchView& bv, int block, in
 {
     const dim3 grid(bv.nblocks, level == 3 ? popcount4(dirmask) : 12);
 #define CALL(R_, L_)                                                                                               \
-    if (level == 1) k_hyp1<N, R_, L_><<<grid, block, 0, s>>>(bv, src, b1, (R_)alpha, nhits, (R_)tol);             \
-    else if (level == 2) k_hyp2<N, R_, L_><<<grid, block, 0, s>>>(bv, src, b1, b2, (R_)alpha, nhits, (R_)tol);    \
+    if (level == 1) k_hyp1<N, R_, L_><<<grid, block, 0, s>>>(bv, src, b1, dirmask, (R_)alpha, nhits, (R_)tol);    \
+    else if (level == 2) k_hyp2<N, R_, L_><<<grid, block, 0, s>>>(bv, src, b1, b2, dirmask, (R_)alpha, nhits, (R_)tol); \
     else k_hyp3<N, R_, L_><<<grid, block, 0, s>>>(bv, src, b2, dst, dirmask, (R_)alpha, nhits, (R_)tol)
     SUN_DISPATCH(fp64, layout, CALL);
 #undef CALL
