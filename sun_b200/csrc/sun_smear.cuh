@@ -104,7 +104,11 @@ template <int N, class R> SUN_DEV R re_tr_nn(const Mat<N, R>& W, const Mat<N, R>
 // the unit element) and multiplied into rows p,q of W; with tol > 0 the hits
 // stop once the relative change of Re tr(W Q)/N is <= tol.  SU3project
 // (projectlink.h:119) is this iteration from W = 1 with tol = 0.
-template <int N, class R> SUN_DEV void project_sun(Mat<N, R>& W, const Mat<N, R>& Q, int nhits, R tol)
+// RSQRT: normalise by rsqrt instead of a square root and a division, a third
+// of a subgroup's chain in FP64.  Only for iterations that tol does not stop:
+// a last-bit change can move the hit at which one stops.
+template <int N, class R, bool RSQRT = false>
+SUN_DEV void project_sun(Mat<N, R>& W, const Mat<N, R>& Q, int nhits, R tol)
 {
     R conver = R(1), old_tr = R(0);
     if (tol > R(0)) old_tr = re_tr_nn(W, Q) / R(N);
@@ -115,9 +119,16 @@ template <int N, class R> SUN_DEV void project_sun(Mat<N, R>& W, const Mat<N, R>
             const int p = SubGroup<N>::p(b), q = SubGroup<N>::q(b);
             R r[4], c[4];
             su2_block_US<N, R>(W, Q, p, q, r);
-            R k = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
-            if (k == R(0)) { k = R(1); r[0] = R(1); }
-            k = R(1) / k;
+            R k;
+            if constexpr (RSQRT) {
+                k = qnorm2(r);
+                if (k == R(0)) r[0] = k = R(1);
+                k = rsqrt(k);
+            } else {
+                k = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
+                if (k == R(0)) { k = R(1); r[0] = R(1); }
+                k = R(1) / k;
+            }
             c[0] = r[0] * k; c[1] = -r[1] * k; c[2] = -r[2] * k; c[3] = -r[3] * k;
             su2_apply<N, R>(W, p, q, c);
         }
@@ -199,8 +210,12 @@ template <class R> SUN_DEV void exp_iq3(const Mat<3, R>& Q, Mat<3, R>& E)
 // APE: U'_mu = P[(U_mu + w S_mu) / (1 + 6 w)], S_mu over the spatial planes --
 // kernel_APE_Space (src/smear/ape.cu:44).  SU(3): SU3project from 1
 // (tol unused); other N: project_link from U_mu with tol.
+// In FP64 the projection's chains bound the kernel (10 hits of three subgroups
+// in sequence, each result 8.6 cycles; the FP64 pipe is two thirds busy).  SU(3)
+// 24^4, copy and three steps: 1.32 ms with a square root and a division per
+// subgroup, 1.18 ms with rsqrt; 1.24 ms capped at 128 registers (four CTAs, spills).
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128) k_ape(BatchView bv, const void* src, void* dst, int dirmask, R w, int nhits,
+__global__ void __launch_bounds__(128, N == 3 && sizeof(R) == 8 ? 3 : 1) k_ape(BatchView bv, const void* src, void* dst, int dirmask, R w, int nhits,
                                              R tol)
 {
     const int b = blockIdx.x;
@@ -225,7 +240,7 @@ __global__ void __launch_bounds__(128) k_ape(BatchView bv, const void* src, void
         }
     if constexpr (N == 3) {
         munit(W);
-        project_sun<N, R>(W, S, nhits, R(0));
+        project_sun<N, R, sizeof(R) == 8>(W, S, nhits, R(0));
     } else {
         W = U;
         project_sun<N, R>(W, S, nhits, tol);
