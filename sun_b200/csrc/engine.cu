@@ -285,7 +285,10 @@ int work_of(const LatDev& L, int kind)
     case WORK_SITES: return L.V;
     case WORK_SPATIAL: return L.X[0] * L.X[1] * L.X[2];
     case WORK_PLANES: return plaquette_items(L.V);
-    case WORK_POLY8: return kPolyLanes * L.X[0] * L.X[1] * L.X[2];
+    case WORK_POLY: {
+        const int V3 = L.X[0] * L.X[1] * L.X[2], spw = 32 / poly_lanes(V3);
+        return 32 * ((V3 + spw - 1) / spw);
+    }
     default: return 4 * L.V;
     }
 }
@@ -594,7 +597,7 @@ void group_plaquette(sun_ctx* c, Group& g, double* out, cudaStream_t s)
 
 void group_polyakov(sun_ctx* c, Group& g, double* out, cudaStream_t s)
 {
-    double* r = group_reduce_fused(g, WORK_POLY8, c->blk_sites, 2, s,
+    double* r = group_reduce_fused(g, WORK_POLY, c->blk_sites, 2, s,
                                    [&](const BatchView& v, double* part, double* out, unsigned* cnt) {
                                        OPS_CALL(g.N, polyakov, g.fp64, g.layout, v, c->blk_sites, part, out, cnt, nullptr, s);
                                    });
@@ -1240,7 +1243,7 @@ static bool solo_measure_graph(sun_lattice* l, Group& g, int n_hb, int n_or, siz
     if (n_hb > 0) upd_view(g, update_block(c, g, MODE_HB, s), s);
     if (n_or > 0) upd_view(g, update_block(c, g, MODE_OR, s), s);
     if (re) g.view(WORK_LINKS, c->blk_links, s);
-    BatchView vp = g.view(WORK_PLANES, c->blk_sites, s), vl = g.view(WORK_POLY8, c->blk_sites, s);
+    BatchView vp = g.view(WORK_PLANES, c->blk_sites, s), vl = g.view(WORK_POLY, c->blk_sites, s);
     // CTAs of 128 threads: the plaquette and the Polyakov loop in one launch
     // (own partials and counters: the two parts run side by side)
     const bool fused = c->blk_sites == 128;
@@ -1322,7 +1325,7 @@ static bool resident_sweeps(sun_lattice* l, Group& g, int n_hb, int n_or, int n_
     }
     if (cap_ctas < 2) return false;
     BatchView upd = upd_view(g, cfg, s);
-    BatchView vp = g.view(WORK_PLANES, 128, s), vl = g.view(WORK_POLY8, 128, s);
+    BatchView vp = g.view(WORK_PLANES, 128, s), vl = g.view(WORK_POLY, 128, s);
     g.partials.ensure(sizeof(double) * 4 * (size_t)(vp.nblocks + vl.nblocks));
     c->res_sync.ensure(4 * sizeof(unsigned));
     c->res_out.ensure(sizeof(double) * 4 * (size_t)n_sweeps);

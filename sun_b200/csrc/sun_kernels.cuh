@@ -818,13 +818,53 @@ SUN_DEV void block_sum(double v, double* out, DD* sh)
     }
     __syncthreads();
 }
+SUN_DEV DD dd_two(double a, double b)
+{
+    DD r;
+    r.s = a + b;
+    const double bb = r.s - a;
+    r.c = (a - (r.s - bb)) + (b - bb);
+    return r;
+}
+SUN_DEV DD dd_shfl_xor(DD d, int o)
+{
+    DD t;
+    t.s = __shfl_xor_sync(0xffffffffu, d.s, o);
+    t.c = __shfl_xor_sync(0xffffffffu, d.c, o);
+    return t;
+}
+// The CTA's sums of two pairs d0, d1: in each warp a butterfly whose first
+// step leaves d0 to one half of the lanes and d1 to the other, then the warps'
+// results in order.  Threads 0 and 1 return the sum of d0 and d1; sh holds
+// two entries per warp.
+SUN_DEV DD cta_sum2(DD d0, DD d1, DD* sh)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const bool hi = lane & 16;
+    DD d = dd_add(hi ? d1 : d0, dd_shfl_xor(hi ? d0 : d1, 16));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) d = dd_add(d, dd_shfl_xor(d, o));
+    if ((lane & 15) == 0) sh[2 * warp + (lane >> 4)] = d;
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        d = sh[threadIdx.x];
+        for (int k = 1; k < nw; ++k) d = dd_add(d, sh[2 * k + threadIdx.x]);
+    }
+    return d;
+}
+// the CTA's sums of v0 and v1 as (sum, compensation) pairs at out[0 .. 3]
+SUN_DEV void block_sum2(double v0, double v1, double* out, DD* sh)
+{
+    const DD d = cta_sum2(DD{v0, 0.0}, DD{v1, 0.0}, sh);
+    if (threadIdx.x < 2) reinterpret_cast<double2*>(out)[threadIdx.x] = make_double2(d.s, d.c);
+    __syncthreads();
+}
 // The sums of CTA partials b0 .. b1 - 1 (two values each), by a whole CTA:
-// thread-strided compensated sums, the shuffle tree of each warp, then the
-// warps' results in order; thread 0 writes value v to dst[v].  (One warp
+// thread-strided compensated sums, then cta_sum2; thread v writes value v to
+// dst[v].  (One warp
 // walking the partials of a 32^4 plaquette, 8,192 CTAs, took 80 us.)
 SUN_DEV void finalize_partials(const double* partials, int b0, int b1, double* dst, DD* sh)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     DD d[2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll 4
     for (int b = b0 + (int)threadIdx.x; b < b1; b += (int)blockDim.x)
@@ -833,17 +873,8 @@ SUN_DEV void finalize_partials(const double* partials, int b0, int b1, double* d
             const double2 p = __ldcg(reinterpret_cast<const double2*>(partials) + 2 * (size_t)b + v);
             d[v] = dd_add(d[v], DD{p.x, p.y});
         }
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-        d[v] = dd_warp(d[v]);
-        if (lane == 0) sh[2 * warp + v] = d[v];
-    }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-        DD t = sh[threadIdx.x];
-        for (int k = 1; k < nw; ++k) t = dd_add(t, sh[2 * k + threadIdx.x]);
-        dst[threadIdx.x] = t.s + t.c;
-    }
+    const DD t = cta_sum2(d[0], d[1], sh);
+    if (threadIdx.x < 2) dst[threadIdx.x] = t.s + t.c;
     __syncthreads();
 }
 // Finalize of lattice l's CTA partials (two values each), run by the last of
@@ -940,69 +971,113 @@ SUN_DEV double plaquette_plane(const LatDev& L, const Geom& g, const int x[4], i
     return mtrace_nd(P, Q).re;
 }
 
-// The six planes of one site of a larger lattice (the values of
-// plaquette_plane).  The site's own links U_1 .. U_3(x), used by three planes
-// each, are widened once and kept in shared memory (element e of U_nu at
-// own[((nu - 1) N N + e) stride]), so 16 links are loaded, rebuilt and widened
-// instead of 24 -- the FP32 -> FP64 conversions, not the FP64 products, would
-// bound the kernel otherwise -- and both products and the trace are formed a
-// row at a time.  N = 6 would take 221 KB per CTA and goes plane by plane.
-template <int N> constexpr bool kPlaquetteOwn = N <= 4;
-template <int N> constexpr int plaquette_smem(int block) { return kPlaquetteOwn<N> ? 3 * N * N * 16 * block : 0; }
+// A link's stored elements on their way from memory: loaded early, rebuilt
+// and widened when needed.
+template <int N, class R, int LAYOUT> struct RawLink {
+    Mat<N, R> F;
+    SUN_DEV void load(const cx<R>* base, uint32_t idx, uint32_t stride)
+    {
+        if constexpr (LAYOUT == L_SOA12) LinkIO<N, R, LAYOUT>::template load_rows<LD_NC>(base, idx, stride, F);
+        else LinkIO<N, R, LAYOUT>::template load<LD_NC>(base, idx, stride, F);
+    }
+    SUN_DEV void widen(Mat<N, double>& A)
+    {
+        if constexpr (LAYOUT == L_SOA12) rebuild12(F);
+        mconvert(F, A);
+    }
+};
+
+// The six planes of one site of a larger lattice.  The site's own links, used
+// by three planes each, are widened once and kept in shared memory (element e
+// of U_mu at own[(mu N N + e) stride]): 16 links are loaded, rebuilt and
+// converted instead of 24.  Both products and the trace are formed a row at a
+// time, the trace in one short chain per row and component (an FP64 result
+// takes 8.6 cycles), and FP32 links of the next plane are loaded before this
+// one is multiplied out, since 12 warps per SM hide too little of an L2 load.
+// 32^4 FP32 12-parameter, cold: 227 us (FP64 pipe 38 %, conversions 30 %), against
+// 278 us with three own links, one load after another and one chain for the
+// trace; products by outer sums at 128 registers (four CTAs) took 304 us.
+// N >= 4 would take 131 KB or more per CTA and goes plane by plane.
+template <int N> constexpr bool kPlaquetteOwn = N <= 3;
+template <int N> constexpr int plaquette_smem(int block) { return kPlaquetteOwn<N> ? 4 * N * N * 16 * block : 0; }
 template <int N, class R, int LAYOUT>
 SUN_DEV void plaquette_site(const LatDev& L, const Geom& g, const int x[4], double2* own, int stride, double& sp,
                             double& tp)
 {
+    constexpr bool kAhead = sizeof(R) == 4;
     const int S[4] = {1, g.X[0], g.X[0] * g.X[1], g.X[0] * g.X[1] * g.X[2]};
     const int lex = lex_of(g, x), par = (x[0] + x[1] + x[2] + x[3]) & 1;
     const cx<R>* base = reinterpret_cast<const cx<R>*>(L.links);
-    auto load = [&](int at, int p, int mu, Mat<N, double>& A) {
-        Mat<N, R> F;
+    auto load = [&](int at, int p, int mu, RawLink<N, R, LAYOUT>& F) {
         const uint32_t s = L.evenodd ? (uint32_t)((at >> 1) + p * g.halfV) : (uint32_t)at;
-        LinkIO<N, R, LAYOUT>::template load<LD_NC>(base, s + (uint32_t)mu * (uint32_t)g.V, 4u * (uint32_t)g.V, F);
-        mconvert(F, A);
+        F.load(base, s + (uint32_t)mu * (uint32_t)g.V, 4u * (uint32_t)g.V);
     };
-    Mat<N, double> A, B, D;
-#pragma unroll 1
-    for (int nu = 1; nu < 4; ++nu) {
-        load(lex, par, nu, B);
+    RawLink<N, R, LAYOUT> FB, FD;
+    // U_nu(x + mu) and U_mu(x + nu) of plane k
+    auto mu_of = [](int k) { return k < 3 ? 0 : (k < 5 ? 1 : 2); };
+    auto nu_of = [](int k) { return k < 3 ? k + 1 : (k < 5 ? k - 1 : 3); };
+    auto load_plane = [&](int k) {
+        const int mu = mu_of(k), nu = nu_of(k);
+        load(lex_step(lex, sel4(x, mu), sel4(g.X, mu), sel4(S, mu), 1), par ^ 1, nu, FB);
+        load(lex_step(lex, sel4(x, nu), sel4(g.X, nu), sel4(S, nu), 1), par ^ 1, mu, FD);
+    };
+    Mat<N, double> B, D;
+    auto keep = [&](int mu) {
 #pragma unroll
         for (int e = 0; e < N * N; ++e)
-            own[((nu - 1) * N * N + e) * stride] = make_double2(B.e[e / N][e % N].re, B.e[e / N][e % N].im);
+            own[(mu * N * N + e) * stride] = make_double2(B.e[e / N][e % N].re, B.e[e / N][e % N].im);
+    };
+    if (kAhead) {
+        RawLink<N, R, LAYOUT> F[4];  // all at once: one memory latency, not four
+#pragma unroll
+        for (int mu = 0; mu < 4; ++mu) load(lex, par, mu, F[mu]);
+        load_plane(0);
+#pragma unroll
+        for (int mu = 0; mu < 4; ++mu) {
+            F[mu].widen(B);
+            keep(mu);
+        }
+    } else {
+#pragma unroll 1
+        for (int mu = 0; mu < 4; ++mu) {
+            load(lex, par, mu, FB);
+            FB.widen(B);
+            keep(mu);
+        }
     }
-    load(lex, par, 0, A);
     sp = 0.0;
     tp = 0.0;
 #pragma unroll 1
-    for (int mu = 0; mu < 3; ++mu) {
-        if (mu > 0) {
+    for (int k = 0; k < 6; ++k) {
+        if (!kAhead) load_plane(k);
+        FB.widen(B);
+        FD.widen(D);
+        if (kAhead && k < 5) load_plane(k + 1);
+        const double2 *ua = own + mu_of(k) * N * N * stride, *uc = own + nu_of(k) * N * N * stride;
+        double re[N], im[N];
 #pragma unroll
-            for (int e = 0; e < N * N; ++e) {
-                const double2 v = own[((mu - 1) * N * N + e) * stride];
-                A.e[e / N][e % N] = mkc(v.x, v.y);
+        for (int i = 0; i < N; ++i) {
+            cx<double> a[N], c[N], p[N], q[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const double2 va = ua[(i * N + j) * stride], vc = uc[(i * N + j) * stride];
+                a[j] = mkc(va.x, va.y);
+                c[j] = mkc(vc.x, vc.y);
+            }
+            rmul<N, double>(a, B, p);
+            rmul<N, double>(c, D, q);
+            re[i] = p[0].re * q[0].re;
+            im[i] = p[0].im * q[0].im;
+#pragma unroll
+            for (int j = 1; j < N; ++j) {
+                re[i] = fma(p[j].re, q[j].re, re[i]);
+                im[i] = fma(p[j].im, q[j].im, im[i]);
             }
         }
-        const int lm = lex_step(lex, sel4(x, mu), sel4(g.X, mu), sel4(S, mu), 1);
-#pragma unroll 1
-        for (int nu = mu + 1; nu < 4; ++nu) {
-            load(lm, par ^ 1, nu, B);
-            load(lex_step(lex, sel4(x, nu), sel4(g.X, nu), sel4(S, nu), 1), par ^ 1, mu, D);
-            double t = 0.0;
+        double t = re[0] + im[0];
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-                cx<double> c[N], p[N], q[N];
-#pragma unroll
-                for (int j = 0; j < N; ++j) {
-                    const double2 v = own[((nu - 1) * N * N + i * N + j) * stride];
-                    c[j] = mkc(v.x, v.y);
-                }
-                rmul<N, double>(A.e[i], B, p);
-                rmul<N, double>(c, D, q);
-#pragma unroll
-                for (int j = 0; j < N; ++j) t = fma(p[j].im, q[j].im, fma(p[j].re, q[j].re, t));
-            }
-            if (nu == 3) tp += t; else sp += t;
-        }
+        for (int i = 1; i < N; ++i) t += re[i] + im[i];
+        if (nu_of(k) == 3) tp += t; else sp += t;
     }
 }
 
@@ -1043,7 +1118,7 @@ SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, d
 }
 
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128) k_plaquette(BatchView bv, double* partials, double* out, unsigned* counters,
+__global__ void __launch_bounds__(128, N <= 3 ? 3 : 1) k_plaquette(BatchView bv, double* partials, double* out, unsigned* counters,
                                                     const unsigned* slot)
 {
     extern __shared__ __align__(16) unsigned char plaquette_raw[];
@@ -1055,8 +1130,7 @@ __global__ void __launch_bounds__(128) k_plaquette(BatchView bv, double* partial
     const int w = (b - __ldg(bv.begin + l)) * blockDim.x + threadIdx.x;
     double sp, tp;
     plaquette_item<N, R, LAYOUT, LD_NC>(L, g, w, sp, tp, reinterpret_cast<double2*>(plaquette_raw));
-    block_sum(sp, partials + (size_t)b * 4, sh);
-    block_sum(tp, partials + (size_t)b * 4 + 2, sh);
+    block_sum2(sp, tp, partials + (size_t)b * 4, sh);
     if (out) finalize_if_last(bv, l, partials, out, counters, slot, sh);
 }
 
@@ -1071,46 +1145,75 @@ template <int N> SUN_DEV void shfl_mat(Mat<N, double>& D, const Mat<N, double>& 
 
 // Polyakov loop -- kernel_calc_polyakovloop_evenodd
 // (src/meas/polyakovloop.cu:54-96): L = U_3(x,0) U_3(x,1) ... U_3(x,T-1),
-// trace summed over spatial sites.  kPolyLanes (8) consecutive lanes per
-// spatial site: lane k multiplies the links t in [k T / 8, (k + 1) T / 8)
-// (an empty range gives the unit matrix), then the lane products are joined
-// in order by a shuffle tree, (P0 P1)(P2 P3)..., so the time chain is T / 8
-// products plus three joins instead of T products.
+// trace summed over spatial sites.  poly_lanes (n) lanes of a warp share a
+// spatial site: lane group k multiplies the links t in [k T / n, (k + 1) T / n)
+// (an empty range gives the unit matrix), then the group products are joined
+// in order by a shuffle tree, (P0 P1)(P2 P3)..., so the time chain is T / n
+// products plus log2 n joins instead of T products.  The 32 / n sites of a
+// warp are consecutive, each group's loads one segment of the image; FP32
+// links are loaded two products ahead.  32^4, cold: 29 us, 49 us with 8 lanes
+// per site and a product with the unit matrix first.
 // Polyakov work item w of lattice L (thread w of k_polyakov's CTAs; all
-// lanes of the warp take part): the trace at the site of lane k == 0, links
-// loaded through path P
+// lanes of the warp take part): the trace at the site of lane group k == 0,
+// links loaded through path P
 template <int N, class R, int LAYOUT, int P>
 SUN_DEV void polyakov_item(const LatDev& L, const Geom& g, int w, double& re, double& im)
 {
+    typedef LinkIO<N, R, LAYOUT> IO;
     const int V3 = g.X[0] * g.X[1] * g.X[2];
-    const int site = w / kPolyLanes, k = w - kPolyLanes * site;
+    const int n = poly_lanes(V3), spw = 32 / n, lane = threadIdx.x & 31;
+    const int site = (w >> 5) * spw + (lane & (spw - 1)), k = lane / spw;
     const bool valid = site < V3;
-    Mat<N, double> Pm, A, T;
+    const cx<R>* base = reinterpret_cast<const cx<R>*>(L.links);
+    const uint32_t mu3 = 3u * (uint32_t)g.V, stride = 4u * (uint32_t)g.V;
+    Mat<N, double> Pm, A;
     munit(Pm);
-    if (valid) {
+    auto times = [&](const Mat<N, double>& B) {  // Pm <- Pm B, a row at a time
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            cx<double> o[N];
+            rmul<N, double>(Pm.e[i], B, o);
+#pragma unroll
+            for (int j = 0; j < N; ++j) Pm.e[i][j] = o[j];
+        }
+    };
+    const int t0 = k * g.X[3] / n, t1 = (k + 1) * g.X[3] / n;
+    if (valid && t1 > t0) {
         int x[4];
         x[0] = site % g.X[0];
         x[1] = (site / g.X[0]) % g.X[1];
         x[2] = site / (g.X[0] * g.X[1]);
-        const int t0 = k * g.X[3] / kPolyLanes, t1 = (k + 1) * g.X[3] / kPolyLanes;
-#pragma unroll 1
-        for (int t = t0; t < t1; ++t) {
-            x[3] = t;
-            load_d<N, R, LAYOUT, P>(L, g, x, 3, A);
-            mmul(Pm, A, T);
-            Pm = T;
-        }
-    }
-    // blockDim is a multiple of 32 and of kPolyLanes: a site's lanes share a
-    // warp, every lane of the warp takes part in the shuffles
-    const int lane = threadIdx.x & 31;
+        x[3] = t0;
+        // image index of U_3(x, t)
+        int lex = lex_of(g, x), par = (x[0] + x[1] + x[2] + t0) & 1;
+        auto index = [&] { return (L.evenodd ? (uint32_t)((lex >> 1) + par * g.halfV) : (uint32_t)lex) + mu3; };
+        constexpr int kAhead = sizeof(R) == 4 ? 2 : 1;
+        Mat<N, R> F[kAhead];
+        auto next = [&](Mat<N, R>& to, int t) {
+            if (t >= t1) return;
+            IO::template load<P>(base, index(), stride, to);
+            lex += V3;
+            par ^= 1;
+        };
+        next(F[0], t0);
+        mconvert(F[0], Pm);
 #pragma unroll
-    for (int step = 1; step < kPolyLanes; step <<= 1) {
-        shfl_mat<N>(A, Pm, lane + step < 32 ? lane + step : lane);
-        if ((k & (2 * step - 1)) == 0) {
-            mmul(Pm, A, T);
-            Pm = T;
-        }
+        for (int i = 0; i < kAhead; ++i) next(F[i], t0 + 1 + i);
+#pragma unroll 1
+        for (int t = t0 + 1; t < t1; t += kAhead)
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i)
+                if (t + i < t1) {
+                    mconvert(F[i], A);
+                    next(F[i], t + i + kAhead);
+                    times(A);
+                }
+    }
+    // every lane of the warp takes part in the shuffles
+#pragma unroll 1
+    for (int step = 1; step < n; step <<= 1) {
+        shfl_mat<N>(A, Pm, lane + step * spw < 32 ? lane + step * spw : lane);
+        if ((k & (2 * step - 1)) == 0) times(A);
     }
     re = 0.0;
     im = 0.0;
@@ -1122,7 +1225,7 @@ SUN_DEV void polyakov_item(const LatDev& L, const Geom& g, int w, double& re, do
 }
 
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128) k_polyakov(BatchView bv, double* partials, double* out, unsigned* counters,
+__global__ void __launch_bounds__(128, N <= 3 ? 4 : 1) k_polyakov(BatchView bv, double* partials, double* out, unsigned* counters,
                                                    const unsigned* slot)
 {
     __shared__ DD sh[32];
@@ -1133,8 +1236,7 @@ __global__ void __launch_bounds__(128) k_polyakov(BatchView bv, double* partials
     const int w = (b - __ldg(bv.begin + l)) * blockDim.x + threadIdx.x;
     double re, im;
     polyakov_item<N, R, LAYOUT, LD_NC>(L, g, w, re, im);
-    block_sum(re, partials + (size_t)b * 4, sh);
-    block_sum(im, partials + (size_t)b * 4 + 2, sh);
+    block_sum2(re, im, partials + (size_t)b * 4, sh);
     if (out) finalize_if_last(bv, l, partials, out, counters, slot, sh);
 }
 
@@ -1146,7 +1248,7 @@ __global__ void __launch_bounds__(128) k_polyakov(BatchView bv, double* partials
 // advances *slot for the next replay and, with end_n_hb >= 0, ends the sweep
 // (the counters, which the measurements do not read).
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128) k_plaq_poly(BatchView vp, BatchView vl, double* part_p, double* part_l,
+__global__ void __launch_bounds__(128, N <= 3 ? 3 : 1) k_plaq_poly(BatchView vp, BatchView vl, double* part_p, double* part_l,
                                                     double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
                                                     unsigned* slot, unsigned* joint, int end_n_hb)
 {
@@ -1163,8 +1265,7 @@ __global__ void __launch_bounds__(128) k_plaq_poly(BatchView vp, BatchView vl, d
     if (plaq) plaquette_item<N, R, LAYOUT, LD_NC>(L, g, w, v0, v1, reinterpret_cast<double2*>(plaquette_raw));
     else polyakov_item<N, R, LAYOUT, LD_NC>(L, g, w, v0, v1);
     double* part = plaq ? part_p : part_l;
-    block_sum(v0, part + (size_t)b * 4, sh);
-    block_sum(v1, part + (size_t)b * 4 + 2, sh);
+    block_sum2(v0, v1, part + (size_t)b * 4, sh);
     const bool fin = finalize_if_last(bv, l, part, plaq ? out_p : out_l, plaq ? cnt_p : cnt_l, slot, sh);
     if (fin && threadIdx.x == 0) {
         __threadfence();
@@ -1193,26 +1294,13 @@ __global__ void __launch_bounds__(128) k_plaq_poly(BatchView vp, BatchView vl, d
 // with host result: 0.71 ms, against 2.99 ms with the lines of every t in
 // local memory, both temporal lines rebuilt for each r (three times the
 // products), a CTA-wide reduction per value and one warp summing 5,184 CTAs.
+// The FP64 pipe is 46 % busy at the 12 warps per SM that the shared memory
+// and the 168 registers allow.
 //
 // (r, t) values leave the warp at once: four (Re and Im of two t's) are
 // reduced together by a compensated butterfly that halves the values as it
 // halves the lanes (11 compensated additions for four values against 20), and
 // added to the warp's sums in shared memory.
-SUN_DEV DD dd_two(double a, double b)
-{
-    DD r;
-    r.s = a + b;
-    const double bb = r.s - a;
-    r.c = (a - (r.s - bb)) + (b - bb);
-    return r;
-}
-SUN_DEV DD dd_shfl_xor(DD d, int o)
-{
-    DD t;
-    t.s = __shfl_xor_sync(0xffffffffu, d.s, o);
-    t.c = __shfl_xor_sync(0xffffffffu, d.c, o);
-    return t;
-}
 // the warp's compensated sums of v0 .. v3: value k in the lanes 8 k .. 8 k + 7
 SUN_DEV DD warp_sum4(double v0, double v1, double v2, double v3)
 {
@@ -1348,7 +1436,7 @@ __global__ void __launch_bounds__(128, WilsonOccupancy<N>::min_blocks) k_wilson(
                     C tr = mkc(0.0, 0.0);
 #pragma unroll
                     for (int i = 0; i < N; ++i) {
-                        C q[N];
+                        C q[N], tri = mkc(0.0, 0.0);  // a row's own chain: an FP64 result takes 8.6 cycles
 #pragma unroll
                         for (int j = 0; j < N; ++j) {
                             const double2 v = Qs[((t - 1) * N * N + i * N + j) * nt];
@@ -1358,8 +1446,9 @@ __global__ void __launch_bounds__(128, WilsonOccupancy<N>::min_blocks) k_wilson(
 #pragma unroll
                         for (int j = 0; j < N; ++j) {
                             Qs[((t - 1) * N * N + i * N + j) * nt] = make_double2(q[j].re, q[j].im);
-                            tr = cfma_nc(K.e[i][j], q[j], tr);
+                            tri = cfma_nc(K.e[i][j], q[j], tri);
                         }
+                        tr = tr + tri;
                     }
                     if (t == t0) w0 = tr;
                     else w1 = tr;
@@ -1743,14 +1832,12 @@ __global__ void __launch_bounds__(128) k_sweeps_resident(ResidentArgs a)
         for (int vb = blockIdx.x; vb < a.plaq.nblocks; vb += gridDim.x) {
             double sp, tp;
             plaquette_item<N, R, LAYOUT, LD_CG>(L, g, vb * (int)blockDim.x + (int)threadIdx.x, sp, tp);
-            block_sum(sp, a.partials + (size_t)vb * 4, sh);
-            block_sum(tp, a.partials + (size_t)vb * 4 + 2, sh);
+            block_sum2(sp, tp, a.partials + (size_t)vb * 4, sh);
         }
         for (int vb = blockIdx.x; vb < a.poly.nblocks; vb += gridDim.x) {
             double re, im;
             polyakov_item<N, R, LAYOUT, LD_CG>(L, g, vb * (int)blockDim.x + (int)threadIdx.x, re, im);
-            block_sum(re, ppart + (size_t)vb * 4, sh);
-            block_sum(im, ppart + (size_t)vb * 4 + 2, sh);
+            block_sum2(re, im, ppart + (size_t)vb * 4, sh);
         }
         if (!cta_arrive(a, done, &seen, first)) return;
         prev = done;

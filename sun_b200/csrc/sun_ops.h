@@ -68,11 +68,14 @@ enum UpdateMode { MODE_HB = 0, MODE_HB_INJECTED = 1, MODE_OR = 2 };
 
 // Work per lattice a launch maps CTAs onto.
 // work items per lattice of a launch: half-sites, sites, spatial sites,
-// links, (site, plane) pairs of the plaquette (6 V), and 8 lanes per spatial
-// site of the Polyakov loop
-enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY8 = 5,
+// links, (site, plane) pairs of the plaquette (6 V), and the lanes of the
+// Polyakov loop's spatial sites (whole warps)
+enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY = 5,
                 WORK_WILSON = 6 };
-constexpr int kPolyLanes = 8;
+// lanes per spatial site of the Polyakov loop: 8 shorten the chain of a small
+// lattice; from kPolyFewV3 spatial sites up there are enough threads with 2
+constexpr int kPolyFewV3 = 8192;
+__host__ __device__ inline int poly_lanes(int V3) { return V3 < kPolyFewV3 ? 8 : 2; }
 // Wilson loops (k_wilson): work items are (tile of `block` consecutive sites,
 // spatial direction), item i = 3 tile + mu, and a CTA takes wilson_per_cta
 // consecutive ones.  kWilsonCtas: the CTAs of one lattice at most -- 3 per SM,
