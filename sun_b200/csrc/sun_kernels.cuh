@@ -260,7 +260,7 @@ template <class R> SUN_DEV cx<R> shfl_cx(cx<R> v, int src)
 
 // Row-split k_update for small lattices of larger N.  The N lanes of a site
 // (32/N sites per warp) each multiply out one row of every staple product,
-// the full neighbour links loaded by every lane (the repeats served by L1);
+// loading their row of its first factor and the whole of the others;
 // the lanes then exchange their rows of the staple sum by warp shuffles, all
 // run the same update on the same inputs, and lane 0 stores the link.  Per
 // lane this holds far fewer live values than one thread per site (SU(6)
@@ -315,7 +315,9 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
     for (int kk = kRot ? 1 : 0; kk < 4; ++kk) {
         const int nu = kRot ? ((mu + kk) & 3) : kk;
         if (!kRot && nu == mu) continue;
-        if (nu == dep) dp.wait();
+        if constexpr (N == 3 && LAYOUT == L_SOA12) {
+            if (nu == dep) dp.wait();
+        }
         const int xn_ = kRot ? sel4(x, nu) : x[kk], Xn_ = kRot ? sel4(g.X, nu) : g.X[kk],
                   Sn_ = kRot ? sel4(st, nu) : st[kk];
         const int lup = lex_step(lex, xn_, Xn_, Sn_, 1);
@@ -366,18 +368,79 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
             mcol<3, R>(A, r, a);
             racc_dn<3, R>(a, B, Sr);
         } else {
-            IO::template load<LD_CG>(base, sx + nu * V, stride, A);
-            IO::template load<LD_CG>(base, syp + mu * V, stride, B);
-            mrow<N, R>(A, r, a);
-            rmul<N, R>(a, B, c);
-            IO::template load<LD_CG>(base, sxpmu + nu * V, stride, A);
-            racc_nd<N, R>(c, A, Sr);
-            IO::template load<LD_CG>(base, sy + nu * V, stride, A);
-            IO::template load<LD_CG>(base, sy + mu * V, stride, B);
-            mcol<N, R>(A, r, a);
-            rmul_dn<N, R>(a, B, c);
-            IO::template load<LD_CG>(base, sz + nu * V, stride, A);
-            racc<N, R>(c, A, Sr);
+            // up: row r of U_nu(x) U_mu(x+nu) U_nu(x+mu)^dagger; down: of
+            // U_nu(x-nu)^dagger U_mu(x-nu) U_nu(x-nu+mu), from row r of the
+            // first factor (column r of the daggered one)
+            cx<R> d[N];
+            Mat<N, R> C;
+            const uint32_t cc = (uint32_t)sx + nu * V, ca = (uint32_t)sxpmu + nu * V, cd = (uint32_t)sy + nu * V,
+                           cz = (uint32_t)sz + nu * V;
+            auto row = [&] {
+                if constexpr (LAYOUT == L_SOA) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) a[k] = ld_elem<R, LD_CG>(base + cc + (uint32_t)(r * N + k) * stride);
+                } else {
+                    Mat<N, R> M;
+                    IO::template load<LD_CG>(base, cc, stride, M);
+                    mrow<N, R>(M, r, a);
+                }
+            };
+            auto col = [&] {
+                if constexpr (LAYOUT == L_SOA) {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) a[k] = ld_elem<R, LD_CG>(base + cd + (uint32_t)(k * N + r) * stride);
+                } else {
+                    Mat<N, R> M;
+                    IO::template load<LD_CG>(base, cd, stride, M);
+                    mcol<N, R>(M, r, a);
+                }
+            };
+            // The previous phase wrote the links of its direction on the sites
+            // of its own parity only: this parity's, or for mu = 0 the other's.
+            // Of the last staples' four links in that direction two are
+            // current, so everything but the products with the other two
+            // comes before the wait.  Not in FP64 overrelaxation, whose
+            // update after the wait is so short that the next launch, which
+            // starts at this wait, would be late (8^4 SU(3): 34.1 against
+            // 28.2 us per pass; heatbath 64.7 with it, 68.1 without).
+            constexpr bool kEarly = MODE != MODE_OR || sizeof(R) == 4;
+            if (kEarly && kRot && kk == 3 && mu != 0) {
+                IO::template load<LD_CG>(base, syp + mu * V, stride, B);
+                IO::template load<LD_CG>(base, ca, stride, A);
+                IO::template load<LD_CG>(base, sy + mu * V, stride, C);
+                col();
+                rmul_dn<N, R>(a, C, d);
+                if (nu == dep) dp.wait();
+                row();
+                IO::template load<LD_CG>(base, cz, stride, C);
+                rmul<N, R>(a, B, c);
+                racc_nd<N, R>(c, A, Sr);
+                racc<N, R>(d, C, Sr);
+            } else if (kEarly && kRot && kk == 3) {
+                IO::template load<LD_CG>(base, syp + mu * V, stride, B);
+                row();
+                rmul<N, R>(a, B, c);
+                IO::template load<LD_CG>(base, sy + mu * V, stride, B);
+                IO::template load<LD_CG>(base, cz, stride, C);
+                if (nu == dep) dp.wait();
+                IO::template load<LD_CG>(base, ca, stride, A);
+                col();
+                racc_nd<N, R>(c, A, Sr);
+                rmul_dn<N, R>(a, B, d);
+                racc<N, R>(d, C, Sr);
+            } else {
+                if (nu == dep) dp.wait();
+                row();
+                IO::template load<LD_CG>(base, syp + mu * V, stride, B);
+                rmul<N, R>(a, B, c);
+                IO::template load<LD_CG>(base, ca, stride, A);
+                racc_nd<N, R>(c, A, Sr);
+                col();
+                IO::template load<LD_CG>(base, sy + mu * V, stride, B);
+                rmul_dn<N, R>(a, B, d);
+                IO::template load<LD_CG>(base, cz, stride, A);
+                racc<N, R>(d, A, Sr);
+            }
         }
     }
 
