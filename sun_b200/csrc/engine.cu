@@ -140,28 +140,21 @@ struct sun_ctx {
     // update kernel: 0 chosen by size (or by the tuner), 1 always one thread
     // per half-site (k_update), 2 always N lanes per half-site (k_update_rows),
     // 3 the tiled kernel where it applies (k_update_tile: N >= 4, full links).
-    // By size: groups of N >= 4, and of SU(3) with FP64 full links, with at
-    // most rows_max_halfv half-sites (FP64: half that) take the row-split
-    // kernel.  Sweeps measured on B200: SU(6) 8^4 FP32 3.1x and FP64 2.2x
-    // faster, 12^4 FP32 1.55x; SU(4) 8^4 16-21 %, 12^4 FP32 10 %; SU(3) FP64
-    // 8^4 5 %.  SU(2), SU(3) in FP32 and larger lattices are faster with one
-    // thread per half-site.
+    // By size: rows_limit.
     int upd_kernel = 0;
     int blk_rows = 128;
     // consecutive update phases launched as programmatic dependents
     // (SUN_B200_PDL=0 turns it off)
     int pdl = 1;
-    long long rows_max_halfv = 16384;
-    // sun_sweep_measure in one cooperative launch (k_sweeps_resident): -1
-    // for SU(3) FP32 lattices of at most resident_max_halfv half-sites, 0
-    // never, 1 whenever the lattice and launch shapes allow
-    // (SUN_B200_RESIDENT).  Measured on B200, 1 HB + 4 OR with both
-    // observables per sweep, us per sweep resident / captured graph: SU(3)
-    // FP32 8^4 188 / 200 (full links), 190 / 189 (12-parameter), 12^4
-    // 206 / 226; slower for FP64 (SU(3) 8^4 230 / 194, 12^4 297 / 268),
-    // SU(2) (8^4 131 / 111), SU(4) (8^4 271 / 224) and from 16^4 up.
-    int resident = -1;
-    long long resident_max_halfv = 16384;
+    long long rows_max_halfv = -1;  // SUN_B200_ROWS_MAX_HALFV (FP64: half of it); -1: rows_limit's own
+    // sun_sweep_measure in cooperative launches (k_sweeps_resident) instead of
+    // a replayed graph: 1 whenever the lattice and launch shapes allow, 0 never
+    // (SUN_B200_RESIDENT; auto: never).  With the row-split kernel's phases
+    // overlapping, the graph is the faster one everywhere.  Measured on B200, 1
+    // HB + 4 OR with both observables per sweep, us per sweep resident / graph:
+    // SU(3) FP32 8^4 205 / 163 (12-parameter), 207 / 148 (full links), 14^4 276
+    // / 239; FP64 8^4 274 / 182.
+    int resident = 0;
     unsigned long long barrier_wait_ns = 1000000000ull;  // one grid barrier wait at most
     int skip_arrive = -1;  // test hook (sun_debug_resident_barrier)
     DevBuf res_sync;       // barrier count, generation, status
@@ -410,6 +403,26 @@ void launch_update(Group& g, int mode, int cfg, const BatchView& v, int par, int
     else OPS_CALL(g.N, update_rows, g.fp64, g.layout, mode, v, -cfg, par, mu, hb_offset, inj, pdl, s);
 }
 
+// The most half-sites (of all the group's lattices) for which the row-split
+// kernel is chosen: it has N times the threads, each with a shorter chain, but
+// more instructions in all, so it wins while the GPU is not full.  Sweeps (1 HB
+// + 4 OR) on B200, us, one thread per half-site / row-split:
+//   SU(3) FP32 full links   8^4 192 / 140, 12^4 209 / 184, 12^3x16 217 / 211, 14^4 231 / 246
+//   SU(3) FP32 12-parameter 4^4 170 / 142, 8^4 178 / 153, 10^4 182 / 164, 12^4 191 / 212
+//   SU(3) FP64 full links   8^4 209 / 175, 10^4 221 / 186, 12^4 231 / 252
+//   SU(4) FP32              8^4 249 / 193, 10^4 264 / 229, 12^4 280 / 300
+//   SU(4) FP64              8^4 339 / 259, 8^3x12 338 / 282, 8^2x12x16 341 / 362
+// FP64 12-parameter links gain nothing (8^4 201 / 200), SU(2) loses (8^4 88 / 142).
+long long rows_limit(const sun_ctx* c, const Group& g)
+{
+    long long own = -1;
+    if (g.N == 3 && g.layout == SUN_SOA) own = g.fp64 ? 7168 : 12288;
+    else if (g.N == 3 && g.layout == SUN_SOA12 && !g.fp64) own = 6144;
+    else if (g.N >= 4) own = g.fp64 ? 4608 : 8192;
+    if (own < 0 || c->rows_max_halfv < 0) return own;
+    return g.fp64 ? c->rows_max_halfv / 2 : c->rows_max_halfv;
+}
+
 // Update launch shape for this group and mode.  Without tuning: by the size
 // rule of sun_ctx::upd_kernel.  With tuning on, the first use of a (class,
 // mode, total half-volume) key times one phase launch per candidate shape on
@@ -425,16 +438,15 @@ int update_block(sun_ctx* c, Group& g, int mode, cudaStream_t s)
         bytes += l->bytes;
     }
     // by size: SU(6) always tiled (1.6-2x faster than one thread per site
-    // from 12^4 up, no spills); small lattices of SU(4) and of SU(3) with
-    // FP64 full links row-split; everything else one thread per half-site
-    const bool small = work <= (g.fp64 ? c->rows_max_halfv / 2 : c->rows_max_halfv);
+    // from 12^4 up, no spills); small lattices row-split (rows_limit);
+    // everything else one thread per half-site
+    const bool small = work <= rows_limit(c, g);
     const int fixed = c->upd_kernel == 1   ? c->blk_update
                       : c->upd_kernel == 2 ? -c->blk_rows
                       : (c->upd_kernel == 3 && tile_ok(g)) ? kCfgTile
                       : (g.N == 6 && tile_ok(g))             ? kCfgTile
-                      : (small && (g.N >= 4 || (g.N == 3 && g.fp64 && g.layout == SUN_SOA)))
-                          ? -c->blk_rows
-                          : c->blk_update;
+                      : small                                ? -c->blk_rows
+                                                             : c->blk_update;
     if (!c->tune) return fixed;
     char key[160];
     snprintf(key, sizeof key, "k_update N=%d %s layout=%d mode=%d halfV=%lld kernel=%d", g.N, g.fp64 ? "f64" : "f32",
@@ -885,8 +897,7 @@ sun_status sun_init(const sun_config* cfg, sun_ctx** out)
             else if (!strcmp(k, "tile")) c->upd_kernel = 3;
         }
         if (const char* t = getenv("SUN_B200_ROWS_MAX_HALFV")) c->rows_max_halfv = atoll(t);
-        if (const char* t = getenv("SUN_B200_RESIDENT")) c->resident = !strcmp(t, "auto") ? -1 : (atoi(t) ? 1 : 0);
-        if (const char* t = getenv("SUN_B200_RESIDENT_MAX_HALFV")) c->resident_max_halfv = atoll(t);
+        if (const char* t = getenv("SUN_B200_RESIDENT")) c->resident = atoi(t) ? 1 : 0;
         if (const char* t = getenv("SUN_B200_PDL")) c->pdl = atoi(t) ? 1 : 0;
         {
             std::lock_guard<std::mutex> lk(g_ctxs_mu);
@@ -1306,7 +1317,6 @@ static bool resident_sweeps(sun_lattice* l, Group& g, int n_hb, int n_or, int n_
     sun_ctx* c = l->ctx;
     const LatDev& L = l->desc;
     if (c->resident == 0 || L.sweep_limit != 0u || c->blk_sites != 128 || g.N > 4) return false;
-    if (c->resident < 0 && (g.N != 3 || g.fp64 || L.halfV > c->resident_max_halfv)) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
     // the launched path's update shapes: one thread per half-site or the

@@ -315,9 +315,6 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
     for (int kk = kRot ? 1 : 0; kk < 4; ++kk) {
         const int nu = kRot ? ((mu + kk) & 3) : kk;
         if (!kRot && nu == mu) continue;
-        if constexpr (N == 3 && LAYOUT == L_SOA12) {
-            if (nu == dep) dp.wait();
-        }
         const int xn_ = kRot ? sel4(x, nu) : x[kk], Xn_ = kRot ? sel4(g.X, nu) : g.X[kk],
                   Sn_ = kRot ? sel4(st, nu) : st[kk];
         const int lup = lex_step(lex, xn_, Xn_, Sn_, 1);
@@ -327,54 +324,104 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
         const int sz = (lex_step(ldn, xm, Xm, Sm, 1) >> 1) + parity * H;
         Mat<N, R> A, B;
         cx<R> a[N], c[N];
+        // The previous phase wrote the links of its direction on the sites of
+        // its own parity only: this parity's, or for mu = 0 the other's.  Of
+        // the last staples' four links in that direction two are current, so
+        // everything but the products with the other two comes before the
+        // wait.  Not in FP64 overrelaxation, whose update after the wait is so
+        // short that the next launch, which starts at this wait, would be late
+        // (8^4 SU(3): 34.1 against 28.2 us per pass; heatbath 64.7 with it,
+        // 68.1 without).
+        constexpr bool kEarly = MODE != MODE_OR || sizeof(R) == 4;
+        const uint32_t cc = (uint32_t)sx + nu * V, cb = (uint32_t)syp + mu * V, ca = (uint32_t)sxpmu + nu * V,
+                       cd = (uint32_t)sy + nu * V, cm = (uint32_t)sy + mu * V, cz = (uint32_t)sz + nu * V;
         if constexpr (N == 3 && LAYOUT == L_SOA12) {
             // up: rows 0, 1 of the two-link product and then of the whole
             // staple by lanes 0, 1 (lane 2 repeats row 0), the staple's row 2
-            // rebuilt from them in every lane
-            cx<R> c0[3], c1[3], c2[3];
-            IO::template load_rows<LD_CG>(base, sx + nu * V, stride, A);
-            IO::template load<LD_CG>(base, syp + mu * V, stride, B);
-            mrow<3, R, 2>(A, r, a);
-            rmul<3, R>(a, B, c);
-            IO::template load<LD_CG>(base, sxpmu + nu * V, stride, A);
-            rmul_nd<3, R>(c, A, a);
+            // rebuilt from them in every lane; down: U_nu(x-nu)^dagger
+            // [U_mu(x-nu) U_nu(x-nu+mu)], the product needed whole
+            const int r01 = r == 1 ? 1 : 0;
+            Mat<N, R> C;
+            cx<R> d[N];
+            auto row = [&](uint32_t at, cx<R> (&o)[N]) {  // a stored row of a link
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                c0[j] = shfl_cx(a[j], lead);
-                c1[j] = shfl_cx(a[j], lead + 1);
+                for (int k = 0; k < 3; ++k) o[k] = ld_elem<R, LD_CG>(base + at + (uint32_t)(r01 * 3 + k) * stride);
+            };
+            auto whole = [&](const cx<R> (&v)[N], cx<R> (&c0)[3], cx<R> (&c1)[3], cx<R> (&c2)[3]) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    c0[j] = shfl_cx(v[j], lead);
+                    c1[j] = shfl_cx(v[j], lead + 1);
+                }
+                rebuild12_row<R>(c0, c1, c2);
+            };
+            auto up = [&] {  // c: row of the two-link product, A = U_nu(x+mu)
+                cx<R> c0[3], c1[3], c2[3];
+                rmul_nd<3, R>(c, A, a);
+                whole(a, c0, c1, c2);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) Sr[j] = Sr[j] + (r == 0 ? c0[j] : (r == 1 ? c1[j] : c2[j]));
+            };
+            auto product = [&](Mat<N, R>& M) {  // d: row of the down product; M the whole of it
+                cx<R> c0[3], c1[3], c2[3];
+                whole(d, c0, c1, c2);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    M.e[0][j] = c0[j];
+                    M.e[1][j] = c1[j];
+                    M.e[2][j] = c2[j];
+                }
+            };
+            if (kEarly && kk == 3 && mu != 0) {
+                IO::template load<LD_CG>(base, cb, stride, B);
+                IO::template load<LD_CG>(base, ca, stride, A);
+                IO::template load<LD_CG>(base, cd, stride, C);
+                cx<R> m[N], col[N];
+                row(cm, m);
+                mcol<3, R>(C, r, col);
+                if (nu == dep) dp.wait();
+                row(cc, a);
+                IO::template load<LD_CG>(base, cz, stride, C);
+                rmul<3, R>(a, B, c);
+                up();
+                rmul<3, R>(m, C, d);
+                product(B);
+                racc_dn<3, R>(col, B, Sr);
+            } else if (kEarly && kk == 3) {
+                IO::template load<LD_CG>(base, cb, stride, B);
+                row(cc, a);
+                rmul<3, R>(a, B, c);
+                row(cm, a);
+                IO::template load<LD_CG>(base, cz, stride, B);
+                rmul<3, R>(a, B, d);
+                product(B);
+                if (nu == dep) dp.wait();
+                IO::template load<LD_CG>(base, ca, stride, A);
+                IO::template load<LD_CG>(base, cd, stride, C);
+                up();
+                mcol<3, R>(C, r, a);
+                racc_dn<3, R>(a, B, Sr);
+            } else {
+                if (nu == dep) dp.wait();
+                row(cc, a);
+                IO::template load<LD_CG>(base, cb, stride, B);
+                rmul<3, R>(a, B, c);
+                IO::template load<LD_CG>(base, ca, stride, A);
+                up();
+                row(cm, a);
+                IO::template load<LD_CG>(base, cz, stride, B);
+                rmul<3, R>(a, B, d);
+                product(B);
+                IO::template load<LD_CG>(base, cd, stride, A);
+                mcol<3, R>(A, r, a);
+                racc_dn<3, R>(a, B, Sr);
             }
-            rebuild12_row<R>(c0, c1, c2);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) Sr[j] = Sr[j] + (r == 0 ? c0[j] : (r == 1 ? c1[j] : c2[j]));
-            // down: U_nu(x-nu)^dagger [U_mu(x-nu) U_nu(x-nu+mu)], the product
-            // needed whole
-            IO::template load_rows<LD_CG>(base, sy + mu * V, stride, A);
-            IO::template load<LD_CG>(base, sz + nu * V, stride, B);
-            mrow<3, R, 2>(A, r, a);
-            rmul<3, R>(a, B, c);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                c0[j] = shfl_cx(c[j], lead);
-                c1[j] = shfl_cx(c[j], lead + 1);
-            }
-            rebuild12_row<R>(c0, c1, c2);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                B.e[0][j] = c0[j];
-                B.e[1][j] = c1[j];
-                B.e[2][j] = c2[j];
-            }
-            IO::template load<LD_CG>(base, sy + nu * V, stride, A);
-            mcol<3, R>(A, r, a);
-            racc_dn<3, R>(a, B, Sr);
         } else {
             // up: row r of U_nu(x) U_mu(x+nu) U_nu(x+mu)^dagger; down: of
             // U_nu(x-nu)^dagger U_mu(x-nu) U_nu(x-nu+mu), from row r of the
             // first factor (column r of the daggered one)
             cx<R> d[N];
             Mat<N, R> C;
-            const uint32_t cc = (uint32_t)sx + nu * V, ca = (uint32_t)sxpmu + nu * V, cd = (uint32_t)sy + nu * V,
-                           cz = (uint32_t)sz + nu * V;
             auto row = [&] {
                 if constexpr (LAYOUT == L_SOA) {
 #pragma unroll
@@ -395,19 +442,10 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
                     mcol<N, R>(M, r, a);
                 }
             };
-            // The previous phase wrote the links of its direction on the sites
-            // of its own parity only: this parity's, or for mu = 0 the other's.
-            // Of the last staples' four links in that direction two are
-            // current, so everything but the products with the other two
-            // comes before the wait.  Not in FP64 overrelaxation, whose
-            // update after the wait is so short that the next launch, which
-            // starts at this wait, would be late (8^4 SU(3): 34.1 against
-            // 28.2 us per pass; heatbath 64.7 with it, 68.1 without).
-            constexpr bool kEarly = MODE != MODE_OR || sizeof(R) == 4;
             if (kEarly && kRot && kk == 3 && mu != 0) {
-                IO::template load<LD_CG>(base, syp + mu * V, stride, B);
+                IO::template load<LD_CG>(base, cb, stride, B);
                 IO::template load<LD_CG>(base, ca, stride, A);
-                IO::template load<LD_CG>(base, sy + mu * V, stride, C);
+                IO::template load<LD_CG>(base, cm, stride, C);
                 col();
                 rmul_dn<N, R>(a, C, d);
                 if (nu == dep) dp.wait();
@@ -417,10 +455,10 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
                 racc_nd<N, R>(c, A, Sr);
                 racc<N, R>(d, C, Sr);
             } else if (kEarly && kRot && kk == 3) {
-                IO::template load<LD_CG>(base, syp + mu * V, stride, B);
+                IO::template load<LD_CG>(base, cb, stride, B);
                 row();
                 rmul<N, R>(a, B, c);
-                IO::template load<LD_CG>(base, sy + mu * V, stride, B);
+                IO::template load<LD_CG>(base, cm, stride, B);
                 IO::template load<LD_CG>(base, cz, stride, C);
                 if (nu == dep) dp.wait();
                 IO::template load<LD_CG>(base, ca, stride, A);
@@ -431,12 +469,12 @@ SUN_DEV void update_rows_warp(const Geom& g, const LatDev& L, int first, int par
             } else {
                 if (nu == dep) dp.wait();
                 row();
-                IO::template load<LD_CG>(base, syp + mu * V, stride, B);
+                IO::template load<LD_CG>(base, cb, stride, B);
                 rmul<N, R>(a, B, c);
                 IO::template load<LD_CG>(base, ca, stride, A);
                 racc_nd<N, R>(c, A, Sr);
                 col();
-                IO::template load<LD_CG>(base, sy + mu * V, stride, B);
+                IO::template load<LD_CG>(base, cm, stride, B);
                 rmul_dn<N, R>(a, B, d);
                 IO::template load<LD_CG>(base, cz, stride, A);
                 racc<N, R>(d, A, Sr);
