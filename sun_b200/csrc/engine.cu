@@ -282,6 +282,7 @@ int work_of(const LatDev& L, int kind)
         const int V3 = L.X[0] * L.X[1] * L.X[2], spw = 32 / poly_lanes(V3);
         return 32 * ((V3 + spw - 1) / spw);
     }
+    case WORK_LINKS8: return (4 * L.V + 7) / 8;
     default: return 4 * L.V;
     }
 }
@@ -503,9 +504,12 @@ int update_block(sun_ctx* c, Group& g, int mode, cudaStream_t s)
     return best;
 }
 
+// the scheduled reunitarization's view: few CTAs, most launches find it not due
+BatchView reunit_view(sun_ctx* c, Group& g, cudaStream_t s) { return g.view(WORK_LINKS8, c->blk_links, s); }
+
 // counters_later: the sweep's counter update is left to the launch after
-// it (the fused measurement of a sweep-and-measure graph; only without a
-// reunitarization, which reads the counters)
+// it (the fused measurement of a sweep-and-measure graph); the
+// reunitarization then reckons with the counters that launch will set
 void group_sweep(sun_ctx* c, Group& g, int n_hb, int n_or, bool count_sweep, bool reunit, cudaStream_t s,
                  bool counters_later = false)
 {
@@ -532,15 +536,15 @@ void group_sweep(sun_ctx* c, Group& g, int n_hb, int n_or, bool count_sweep, boo
                 for (int mu = 0; mu < 4; ++mu, pdl = c->pdl)
                     launch_update(g, MODE_OR, bor, vor, par, mu, 0u, none, s, pdl);
     }
-    if ((n_hb > 0 || count_sweep) && !(counters_later && !reunit))
+    if ((n_hb > 0 || count_sweep) && !counters_later)
         ck(launch_end_sweep(reinterpret_cast<const LatDev*>(g.d_lats.p), (int)g.lats.size(), (unsigned)n_hb,
                             count_sweep ? 1u : 0u, s),
            "end_sweep");
     // end_sweep above also bumped the sweep counter when count_sweep; the
     // reunitarization kernel checks each lattice's own schedule on device
     if (reunit) {
-        BatchView links = g.view(WORK_LINKS, c->blk_links, s);
-        OPS_CALL(g.N, reunit, g.fp64, g.layout, links, c->blk_links, 1, s);
+        OPS_CALL(g.N, reunit, g.fp64, g.layout, reunit_view(c, g, s), c->blk_links,
+                 counters_later ? REUNIT_DUE_NEXT : REUNIT_DUE, s);
     }
 }
 
@@ -1177,7 +1181,7 @@ static bool solo_sweep_graph(sun_lattice* l, Group& g, int n_hb, int n_or, bool 
     // launch shapes (tuned if tuning is on) and their tables, before capture
     if (n_hb > 0) upd_view(g, update_block(l->ctx, g, MODE_HB, s), s);
     if (n_or > 0) upd_view(g, update_block(l->ctx, g, MODE_OR, s), s);
-    if (re) g.view(WORK_LINKS, l->ctx->blk_links, s);
+    if (re) reunit_view(l->ctx, g, s);
     cudaStream_t cs;
     ck(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream");
     cudaGraph_t graph;
@@ -1253,7 +1257,7 @@ static bool solo_measure_graph(sun_lattice* l, Group& g, int n_hb, int n_or, siz
     // launch shapes, tables and scratch before the capture
     if (n_hb > 0) upd_view(g, update_block(c, g, MODE_HB, s), s);
     if (n_or > 0) upd_view(g, update_block(c, g, MODE_OR, s), s);
-    if (re) g.view(WORK_LINKS, c->blk_links, s);
+    if (re) reunit_view(c, g, s);
     BatchView vp = g.view(WORK_PLANES, c->blk_sites, s), vl = g.view(WORK_POLY, c->blk_sites, s);
     // CTAs of 128 threads: the plaquette and the Polyakov loop in one launch
     // (own partials and counters: the two parts run side by side)
@@ -1281,7 +1285,7 @@ static bool solo_measure_graph(sun_lattice* l, Group& g, int n_hb, int n_or, siz
         if (fused) {
             unsigned* mc = reinterpret_cast<unsigned*>(l->meas_cnt.p);
             OPS_CALL(g.N, plaq_poly, g.fp64, g.layout, vp, g.large(), vl, part, part + 4 * (size_t)vp.nblocks, out_p, out_l, mc,
-                     mc + 1, slot, mc + 2, re ? -1 : n_hb, cs);
+                     mc + 1, slot, mc + 2, n_hb, cs);
         } else {
             OPS_CALL(g.N, plaquette, g.fp64, g.layout, vp, g.large(), c->blk_sites, part, out_p, cnt, slot, cs);
             OPS_CALL(g.N, polyakov, g.fp64, g.layout, vl, c->blk_sites, part, out_l, cnt, slot, cs);
@@ -1448,7 +1452,7 @@ sun_status sun_reunitarize(sun_lattice* l, void* stream)
         cudaStream_t s = S(l->ctx, stream);
         Solo so(l);
         BatchView v = so.g.view(WORK_LINKS, l->ctx->blk_links, s);
-        OPS_CALL(l->p.ncolors, reunit, so.g.fp64, so.g.layout, v, l->ctx->blk_links, 0, s);
+        OPS_CALL(l->p.ncolors, reunit, so.g.fp64, so.g.layout, v, l->ctx->blk_links, REUNIT_ALL, s);
         ck(cudaStreamSynchronize(s), "reunitarize");
     });
 }
@@ -1875,7 +1879,7 @@ sun_status sun_batch_sweep(sun_batch* b, int n_hb, int n_or, int n_sweeps, int u
                 if (g->lats.empty()) continue;
                 if (n_hb > 0) upd_view(*g, update_block(b->ctx, *g, MODE_HB, s), s);
                 if (n_or > 0) upd_view(*g, update_block(b->ctx, *g, MODE_OR, s), s);
-                g->view(WORK_LINKS, b->ctx->blk_links, s);
+                reunit_view(b->ctx, *g, s);
             }
             for (int i = 0; i < n_sweeps; ++i) batch_one_sweep(b, n_hb, n_or, s, true);
             if (wait) ck(cudaStreamSynchronize(s), "batch sweep");
@@ -1889,7 +1893,7 @@ sun_status sun_batch_sweep(sun_batch* b, int n_hb, int n_or, int n_sweeps, int u
                 // launch shapes (tuned if tuning is on) and their tables, before capture
                 if (n_hb > 0) upd_view(*g, update_block(b->ctx, *g, MODE_HB, s), s);
                 if (n_or > 0) upd_view(*g, update_block(b->ctx, *g, MODE_OR, s), s);
-                g->view(WORK_LINKS, b->ctx->blk_links, s);
+                reunit_view(b->ctx, *g, s);
             }
             cudaStream_t cs;
             ck(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream");

@@ -860,21 +860,21 @@ template <int N, class R, int LAYOUT, int P> SUN_DEV void reunit_link(const LatD
     LinkIO<N, R, LAYOUT>::store(base, (uint32_t)w, 4u * L.V, U);
 }
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(256) k_reunit(BatchView bv, int only_due)
+__global__ void __launch_bounds__(256) k_reunit(BatchView bv, ReunitWhen when)
 {
     const int b = blockIdx.x;
     const int l = find_lat(bv, b);
     const LatDev& L = bv.lats[l];
-    if (only_due) {
+    if (when != REUNIT_ALL) {
         // due after a sweep that advanced the lattice (not after the sweeps
         // a lattice at its sweep limit sits out)
-        if (L.reunit_every <= 0 || L.state[2] == 0u) return;
-        const unsigned sw = L.state[1];
-        if (sw == 0u || (sw % (unsigned)L.reunit_every) != 0u) return;
+        if (L.reunit_every <= 0) return;
+        const bool adv = when == REUNIT_DUE ? L.state[2] != 0u : L.sweep_limit == 0u || L.state[1] < L.sweep_limit;
+        const unsigned sw = L.state[1] + (when == REUNIT_DUE_NEXT);
+        if (!adv || sw == 0u || (sw % (unsigned)L.reunit_every) != 0u) return;
     }
-    const int w = (b - __ldg(bv.begin + l)) * blockDim.x + threadIdx.x;
-    if (w >= 4 * L.V) return;
-    reunit_link<N, R, LAYOUT, LD_CA>(L, w);
+    const int b0 = __ldg(bv.begin + l), step = (__ldg(bv.begin + l + 1) - b0) * blockDim.x;
+    for (int w = (b - b0) * blockDim.x + threadIdx.x; w < 4 * L.V; w += step) reunit_link<N, R, LAYOUT, LD_CA>(L, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -1916,7 +1916,7 @@ __global__ void __launch_bounds__(128) k_sweeps_resident(ResidentArgs a)
                     done += P;
                 }
         }
-        // reunitarization on the lattice's schedule, as k_reunit(only_due)
+        // reunitarization on the lattice's schedule, as k_reunit
         const unsigned swn = sweeps0 + (unsigned)sw + 1u;
         if (L.reunit_every > 0 && swn % (unsigned)L.reunit_every == 0u) {
             if (!cta_wait(a, done, &seen)) return;
@@ -2119,9 +2119,9 @@ template <int N> cudaError_t Ops<N>::hot(int fp64, int layout, const BatchView& 
 }
 
 template <int N>
-cudaError_t Ops<N>::reunit(int fp64, int layout, const BatchView& bv, int block, int only_due, cudaStream_t s)
+cudaError_t Ops<N>::reunit(int fp64, int layout, const BatchView& bv, int block, ReunitWhen when, cudaStream_t s)
 {
-#define CALL(R_, L_) k_reunit<N, R_, L_><<<bv.nblocks, block, 0, s>>>(bv, only_due)
+#define CALL(R_, L_) k_reunit<N, R_, L_><<<bv.nblocks, block, 0, s>>>(bv, when)
     SUN_DISPATCH(fp64, layout, CALL);
 #undef CALL
     return cudaGetLastError();

@@ -63,15 +63,19 @@ struct InjView {
     int* err;
 };
 
+// which lattices a reunitarization launch works on: all; those due by their
+// sweep counters; those that will be due once the sweep just run is counted
+enum ReunitWhen { REUNIT_ALL = 0, REUNIT_DUE = 1, REUNIT_DUE_NEXT = 2 };
+
 enum UpdateMode { MODE_HB = 0, MODE_HB_INJECTED = 1, MODE_OR = 2 };
 
 
 // Work per lattice a launch maps CTAs onto.
 // work items per lattice of a launch: half-sites, sites, spatial sites,
-// links, (site, plane) pairs of the plaquette (6 V), and the lanes of the
-// Polyakov loop's spatial sites (whole warps)
+// links (8 per thread: LINKS8), (site, plane) pairs of the plaquette (6 V), and
+// the lanes of the Polyakov loop's spatial sites (whole warps)
 enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY = 5,
-                WORK_WILSON = 6 };
+                WORK_WILSON = 6, WORK_LINKS8 = 7 };
 // lanes per spatial site of the Polyakov loop: 8 shorten the chain of a small
 // lattice; from kPolyFewV3 spatial sites up there are enough threads with 2
 constexpr int kPolyFewV3 = 8192;
@@ -158,10 +162,9 @@ template <int N> struct Ops {
     static int resident_capacity(int fp64, int layout, int rows);
     static cudaError_t cold(int fp64, int layout, const BatchView& bv, int block, cudaStream_t s);
     static cudaError_t hot(int fp64, int layout, const BatchView& bv, int block, cudaStream_t s);
-    // FP64 reunitarization; only_due: skip lattices whose sweep counter is not
-    // a multiple of reunit_every
-    static cudaError_t reunit(int fp64, int layout, const BatchView& bv, int block, int only_due,
-                              cudaStream_t s);
+    // FP64 reunitarization of the lattices that `when` selects; the view may
+    // hold fewer threads than links
+    static cudaError_t reunit(int fp64, int layout, const BatchView& bv, int block, ReunitWhen when, cudaStream_t s);
     // per-CTA partials: plaquette 2 values, polyakov 2, unitarity 1 (max);
     // partial layout [block][value][sum, compensation]
     // plaquette and polyakov: with out non-null, the last CTA of each
