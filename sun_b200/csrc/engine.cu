@@ -271,13 +271,13 @@ public:
 
 cudaStream_t S(sun_ctx* c, void* s) { return s ? reinterpret_cast<cudaStream_t>(s) : c->stream; }
 
-int work_of(const LatDev& L, int kind)
+int work_of(const LatDev& L, int N, int kind)
 {
     switch (kind) {
     case WORK_HALF: return L.halfV;
     case WORK_SITES: return L.V;
     case WORK_SPATIAL: return L.X[0] * L.X[1] * L.X[2];
-    case WORK_PLANES: return plaquette_items(L.V);
+    case WORK_PLANES: return plaquette_items(N, L.V);
     case WORK_POLY: {
         const int V3 = L.X[0] * L.X[1] * L.X[2], spw = 32 / poly_lanes(V3);
         return 32 * ((V3 + spw - 1) / spw);
@@ -287,13 +287,13 @@ int work_of(const LatDev& L, int kind)
     }
 }
 
-int ctas_of(const LatDev& L, int kind, int block)
+int ctas_of(const LatDev& L, int N, int kind, int block)
 {
     if (kind == WORK_WILSON) {
         const int per = wilson_per_cta(L.V, block);
         return (wilson_items(L.V, block) + per - 1) / per;
     }
-    return (work_of(L, kind) + block - 1) / block;
+    return (work_of(L, N, kind) + block - 1) / block;
 }
 
 // Same-class lattices advanced by one launch per kernel.
@@ -318,7 +318,7 @@ struct Group {
     int large() const
     {
         for (auto* l : lats)
-            if (l->desc.V >= kPlaneSplitMaxV) return 1;
+            if (l->desc.V >= plane_split_max_v(N)) return 1;
         return 0;
     }
 
@@ -350,7 +350,7 @@ struct Group {
         if (!e.valid) {
             std::vector<int> b(lats.size() + 1, 0);
             for (size_t i = 0; i < lats.size(); ++i)
-                b[i + 1] = b[i] + ctas_of(lats[i]->desc, kind, block);
+                b[i + 1] = b[i] + ctas_of(lats[i]->desc, N, kind, block);
             if (!e.buf) e.buf = std::make_shared<DevBuf>();
             e.buf->ensure(sizeof(int) * b.size());
             ck(cudaMemcpyAsync(e.buf->p, b.data(), sizeof(int) * b.size(), cudaMemcpyHostToDevice, s), "begin upload");
@@ -1321,6 +1321,7 @@ static bool resident_sweeps(sun_lattice* l, Group& g, int n_hb, int n_or, int n_
     sun_ctx* c = l->ctx;
     const LatDev& L = l->desc;
     if (c->resident == 0 || L.sweep_limit != 0u || c->blk_sites != 128 || g.N > 4) return false;
+    if (L.V >= plane_split_max_v(g.N)) return false;  // their plaquette (plaquette_site) has no resident form
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
     // the launched path's update shapes: one thread per half-site or the

@@ -1049,7 +1049,7 @@ SUN_DEV void load_d(const LatDev& L, const Geom& g, const int x[4], int mu, Mat<
 // (src/meas/plaquette_cub.cu:47-145): per site sum over mu < nu of
 // Re tr[U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag], nu == 3 temporal.
 // Links are widened to FP64 before the products.  Lattices below
-// kPlaneSplitMaxV sites take one thread per (site, plane), warp-major (a
+// plane_split_max_v sites take one thread per (site, plane), warp-major (a
 // warp holds one plane of 32 consecutive sites, so its loads coalesce): a
 // small lattice's launch then lasts one plaquette instead of six.  Larger
 // lattices take one thread per site.  Sites are walked in lexicographic
@@ -1190,7 +1190,7 @@ SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, d
 {
     sp = 0.0;
     tp = 0.0;
-    if (g.V < kPlaneSplitMaxV) {
+    if (g.V < plane_split_max_v(N)) {
         const int chunk = w / 192, r = w - 192 * chunk, plane = r >> 5;
         const int site = chunk * 32 + (r & 31);
         if (site < g.V) {

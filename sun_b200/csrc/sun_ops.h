@@ -110,9 +110,16 @@ __host__ __device__ inline int wilson_block(int N, int R, int T)
 }
 // lattices below this volume measure the plaquette with one thread per
 // (site, plane), warp-major (a warp: one plane of 32 consecutive sites), the
-// others with one thread per site; the choice depends on the lattice alone
-constexpr int kPlaneSplitMaxV = 1 << 17;
-__host__ __device__ inline int plaquette_items(int V) { return V < kPlaneSplitMaxV ? ((V + 31) / 32) * 192 : V; }
+// others with one thread per site; the choice depends on the lattice alone.
+// N <= 3: a site's thread loads and converts two thirds of the links that its
+// planes' threads would, and from 2^15 sites there are enough of them (sun_plaquette
+// of SU(3), us, planes / sites: 14^4 FP32 32.2 / 26.9, FP64 36.0 / 30.1; 16^4 41.0
+// / 31.2 and 45.6 / 36.3; 16^3x24 54.7 / 38.0 and 61.2 / 43.3).
+__host__ __device__ constexpr int plane_split_max_v(int N) { return N <= 3 ? 1 << 15 : 1 << 17; }
+__host__ __device__ inline int plaquette_items(int N, int V)
+{
+    return V < plane_split_max_v(N) ? ((V + 31) / 32) * 192 : V;
+}
 
 // Many sweeps of one lattice in one cooperative launch (k_sweeps_resident):
 // the update phases, the reunitarization and the measurements separated by
@@ -171,7 +178,7 @@ template <int N> struct Ops {
     // lattice also finalizes its sums into out[2 l .. 2 l + 1] (counters: one
     // zeroed unsigned per lattice, left at zero); with slot non-null, into
     // row *slot of out (2 nlat doubles per row)
-    // large: a lattice of the view has at least kPlaneSplitMaxV sites
+    // large: a lattice of the view has at least plane_split_max_v(N) sites
     static cudaError_t plaquette(int fp64, int layout, const BatchView& bv, int large, int block, double* partials,
                                  double* out, unsigned* counters, const unsigned* slot, cudaStream_t s);
     static cudaError_t polyakov(int fp64, int layout, const BatchView& bv, int block, double* partials,
