@@ -1210,6 +1210,10 @@ static void solo_passes(sun_lattice* l, int n_hb, int n_or, int n_sweeps, bool c
     need_eo(l, "the heatbath/overrelaxation update");
     Solo so(l);
     const bool re = count && l->p.reunit_every > 0;
+    // the table a later captured sweep needs, with the update's own
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (l->p.reunit_every > 0 && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+        reunit_view(l->ctx, so.g, s);
     if (count && n_sweeps > 0 && solo_sweep_graph(l, so.g, n_hb, n_or, re, s)) {
         for (int i = 0; i < n_sweeps; ++i) ck(cudaGraphLaunch(l->sweep_graph, s), "graph launch");
         return;

@@ -9,6 +9,8 @@
 #include "sun_core.cuh"
 #include "sun_ops.h"
 
+#include <atomic>
+
 namespace sunb {
 
 SUN_DEV int find_lat(const BatchView& bv, int b)
@@ -2023,6 +2025,20 @@ cudaError_t Ops<N>::update_rows(int fp64, int layout, int mode, const BatchView&
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+// Opts a kernel in to `bytes` of dynamic shared memory, once per device.
+template <auto KERNEL> cudaError_t allow_smem(int bytes)
+{
+    static std::atomic<unsigned long long> done{0ull};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (done.load() & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit);
+    return e;
+}
+
 // the tiled update's instance for (R, MODE), its shared memory opted in once
 template <int N, class R, int MODE> cudaError_t launch_tile(const BatchView& bv, int parity, int mu,
                                                             unsigned hb_offset, const InjView& inj, int pdl,
@@ -2032,11 +2048,10 @@ template <int N, class R, int MODE> cudaError_t launch_tile(const BatchView& bv,
     // the dynamic size opted in above 48 KB.  The shared-memory carve-out is
     // left to the driver: forcing the largest one measured slower (SU(6)
     // 24^4 FP64 21.7 -> 38.0 ms per sweep, FP32 9.6 -> 10.7 ms).
-    static const cudaError_t attr =
-        smem > 48 * 1024
-            ? cudaFuncSetAttribute(k_update_tile<N, R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-            : cudaSuccess;
-    if (attr != cudaSuccess) return attr;
+    if (smem > 48 * 1024) {
+        const cudaError_t attr = allow_smem<k_update_tile<N, R, MODE>>(smem);
+        if (attr != cudaSuccess) return attr;
+    }
     return launch_phase(k_update_tile<N, R, MODE>, bv, 32 * N / tile_rpw<N, R>(), parity, mu, hb_offset, inj, pdl, s,
                         smem);
 }
@@ -2127,15 +2142,6 @@ cudaError_t Ops<N>::reunit(int fp64, int layout, const BatchView& bv, int block,
     return cudaGetLastError();
 }
 
-// the shared memory of a large lattice's plaquette (above 48 KB for N >= 3),
-// opted in once per instance
-template <int N, auto KERNEL> cudaError_t allow_plaquette_smem()
-{
-    static const cudaError_t e =
-        cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, plaquette_smem<N>(128));
-    return e;
-}
-
 template <int N>
 cudaError_t Ops<N>::plaquette(int fp64, int layout, const BatchView& bv, int large, int block, double* partials,
                               double* out, unsigned* counters, const unsigned* slot, cudaStream_t s)
@@ -2143,7 +2149,7 @@ cudaError_t Ops<N>::plaquette(int fp64, int layout, const BatchView& bv, int lar
     const int smem = large ? plaquette_smem<N>(block) : 0;
     cudaError_t e = cudaSuccess;
 #define CALL(R_, L_)                                                                                        \
-    if ((e = allow_plaquette_smem<N, k_plaquette<N, R_, L_>>()) == cudaSuccess)                               \
+    if ((e = smem ? allow_smem<k_plaquette<N, R_, L_>>(plaquette_smem<N>(128)) : cudaSuccess) == cudaSuccess)                               \
         k_plaquette<N, R_, L_><<<bv.nblocks, block, smem, s>>>(bv, partials, out, counters, slot)
     SUN_DISPATCH(fp64, layout, CALL);
 #undef CALL
@@ -2168,7 +2174,7 @@ cudaError_t Ops<N>::plaq_poly(int fp64, int layout, const BatchView& vp, int lar
     const int smem = large ? plaquette_smem<N>(128) : 0;
     cudaError_t e = cudaSuccess;
 #define CALL(R_, L_)                                                                                            \
-    if ((e = allow_plaquette_smem<N, k_plaq_poly<N, R_, L_>>()) == cudaSuccess)                                   \
+    if ((e = smem ? allow_smem<k_plaq_poly<N, R_, L_>>(plaquette_smem<N>(128)) : cudaSuccess) == cudaSuccess)                                   \
         k_plaq_poly<N, R_, L_><<<vp.nblocks + vl.nblocks, 128, smem, s>>>(vp, vl, part_p, part_l, out_p, out_l, \
                                                                           cnt_p, cnt_l, slot, joint, end_n_hb)
     SUN_DISPATCH(fp64, layout, CALL);
@@ -2176,13 +2182,12 @@ cudaError_t Ops<N>::plaq_poly(int fp64, int layout, const BatchView& vp, int lar
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// the instance's shared memory is opted in once, at the most any R, T <= 8 takes
+// the instance's shared memory is opted in at the most any R, T <= 8 takes
 template <int N, class R, int LAYOUT>
 cudaError_t launch_wilson(const BatchView& bv, int RR, int TT, double2* partials, cudaStream_t s)
 {
     const int block = wilson_block(N, RR, TT), smem = wilson_smem(N, RR, TT, block);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_wilson<N, R, LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    const cudaError_t attr = allow_smem<k_wilson<N, R, LAYOUT>>(160 * 1024);
     static_assert(16 * (32 * SUN_WMAX * N * N + 2 * SUN_WMAX * SUN_WMAX + 2 * SUN_WMAX) <= 160 * 1024, "");
     if (attr != cudaSuccess) return attr;
     k_wilson<N, R, LAYOUT><<<bv.nblocks, block, smem, s>>>(bv, RR, TT, partials);
