@@ -1542,17 +1542,27 @@ void check_dirmask(int dirmask)
     if (dirmask <= 0 || dirmask > 15) fail(SUN_ERR_INVALID_ARG, "direction mask %d not in 1..15", dirmask);
 }
 
-// the links of the directions in dirmask, from one image of l to another
+// the links of the directions in dirmask, from one image of l to another: a
+// pitched copy per run of directions, or, where the pitch (the four directions
+// of one element) is above the device's documented limit for it (2^31 - 1 bytes:
+// from 2^25 sites in FP64, 2^26 in FP32), a plain copy per element and run
 void copy_directions(sun_lattice* l, void* dst, const void* src, int dirmask, cudaStream_t s)
 {
     const size_t csz = l->p.precision == SUN_F64 ? 16 : 8, row = csz * (size_t)l->desc.V;  // one direction of one element
+    const int elems = elems_of(l->p.ncolors, l->p.layout);
+    int max_pitch = 0;
+    ck(cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, l->ctx->device), "max pitch");
     for (int mu = 0; mu < 4;) {
         int n = 0;
         while (mu + n < 4 && ((dirmask >> (mu + n)) & 1)) ++n;
-        if (n)
-            ck(cudaMemcpy2DAsync((char*)dst + mu * row, 4 * row, (const char*)src + mu * row, 4 * row, n * row,
-                                 elems_of(l->p.ncolors, l->p.layout), cudaMemcpyDeviceToDevice, s),
-               "smear scratch");
+        char* d = (char*)dst + mu * row;
+        const char* f = (const char*)src + mu * row;
+        if (n && 4 * row <= (size_t)max_pitch)
+            ck(cudaMemcpy2DAsync(d, 4 * row, f, 4 * row, n * row, elems, cudaMemcpyDeviceToDevice, s), "smear scratch");
+        else if (n)
+            for (int e = 0; e < elems; ++e)
+                ck(cudaMemcpyAsync(d + 4 * row * e, f + 4 * row * e, n * row, cudaMemcpyDeviceToDevice, s),
+                   "smear scratch");
         mu += n + 1;
     }
 }
