@@ -83,6 +83,12 @@ const char *sun_last_error_string(const sun_ctx *ctx);
 /* the context's device-memory admission budget: sun_config.hbm_budget_bytes,
  * or 90% of the free memory at sun_init; servers admit jobs against it */
 sun_status sun_ctx_hbm_budget(const sun_ctx *ctx, size_t *bytes);
+/* frees the scratch images that the context keeps between calls: up to 2 GB of
+ * device memory after smearing, conversions between layouts and canonical
+ * uploads or downloads, outside the budget above.  They are also freed with the
+ * context, and by the library when one of its own allocations fails; call this
+ * before other users of the device need the memory */
+sun_status sun_ctx_release_scratch(sun_ctx *ctx);
 const char *sun_version(void);
 /* host-side fault injection for tests (no reference counterpart): after
  * after_n more device allocations succeed, every further one reports

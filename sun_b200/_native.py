@@ -74,6 +74,7 @@ _SIGS = {
     "sun_lattice_set_rng": [_vp, C.c_uint64, C.c_uint32, C.c_uint32],
     "sun_lattice_set_sweep_limit": [_vp, C.c_uint32],
     "sun_ctx_hbm_budget": [_vp, C.POINTER(C.c_size_t)],
+    "sun_ctx_release_scratch": [_vp],
     "sun_heatbath": [_vp, C.c_int, _vp],
     "sun_overrelax": [_vp, C.c_int, _vp],
     "sun_sweep": [_vp, C.c_int, C.c_int, C.c_int, _vp],

@@ -62,6 +62,10 @@ class Context:
             lib().sun_finalize(self.h)
             self.h = None
 
+    def release_scratch(self) -> None:
+        """Free the scratch images kept between calls (up to 2 GB)."""
+        check(lib().sun_ctx_release_scratch(self.h), self.h)
+
     def __enter__(self):
         return self
 

@@ -159,8 +159,8 @@ struct sun_ctx {
     int skip_arrive = -1;  // test hook (sun_debug_resident_barrier)
     DevBuf res_sync;       // barrier count, generation, status
     DevBuf res_out;        // per-sweep plaquette and Polyakov sums
-    // scratch images kept between calls (ScratchLease), freed with the context
-    // or when an allocation fails
+    // scratch images kept between calls (ScratchLease), freed with the context,
+    // by sun_ctx_release_scratch, or when an allocation of the library fails
     std::vector<std::unique_ptr<DevBuf>> kept;
     // autotuner (tuneLaunch, src/tune.cpp:304): CTA size of the update kernel
     // per (kernel class, total half-volume), timed once, cached in a CSV file
@@ -202,20 +202,20 @@ struct sun_lattice {
 
 namespace {
 
-// every live context, for release_kept_scratch
-std::mutex g_ctxs_mu;
+// guards every context's kept scratch, and the list of live contexts
+std::mutex g_kept_mu;
 std::vector<sun_ctx*> g_ctxs;
 
+// kept buffers are in no call's use, so a context busy in another thread gives
+// its own too
 bool release_kept_scratch()
 {
     bool any = false;
-    std::lock_guard<std::mutex> lk(g_ctxs_mu);
-    for (sun_ctx* c : g_ctxs)
-        if (c->mu.try_lock()) {  // another thread's context in a call keeps its scratch
-            any |= !c->kept.empty();
-            c->kept.clear();
-            c->mu.unlock();
-        }
+    std::lock_guard<std::mutex> lk(g_kept_mu);
+    for (sun_ctx* c : g_ctxs) {
+        any |= !c->kept.empty();
+        c->kept.clear();
+    }
     return any;
 }
 
@@ -223,9 +223,10 @@ bool release_kept_scratch()
 // canonical copy of a conversion).  A cudaMalloc and cudaFree of these sizes
 // cost more than the work on them (SU(3) 24^4: APE in FP64 1 ms of 3 ms, HYP in
 // FP32 2.5 ms of 4.7 ms per call), so up to kScratchKeep bytes stay with the
-// context for the next call.  Calls that lease scratch hold the context's lock
-// and synchronise their stream before they return, so no two ever use a buffer
-// at once, whatever their streams; a call that throws synchronises here.
+// context for the next call (sun_ctx_release_scratch gives them back).  Calls
+// that lease scratch hold the context's lock and synchronise their stream
+// before they return, so no two ever use a buffer at once, whatever their
+// streams; a call that throws synchronises here.
 constexpr size_t kScratchKeep = (size_t)2 << 30;
 class ScratchLease {
     sun_ctx* c;
@@ -233,27 +234,20 @@ class ScratchLease {
     int exceptions = std::uncaught_exceptions();
     std::vector<std::unique_ptr<DevBuf>> bufs;
 
-public:
-    ScratchLease(sun_ctx* c_, cudaStream_t s_) : c(c_), s(s_) {}
-    ScratchLease(const ScratchLease&) = delete;
-    void* get(size_t bytes)
+    std::unique_ptr<DevBuf> take(size_t bytes)  // the smallest kept buffer that is large enough, if any
     {
+        std::lock_guard<std::mutex> lk(g_kept_mu);
         auto best = c->kept.end();
         for (auto it = c->kept.begin(); it != c->kept.end(); ++it)
             if ((*it)->n >= bytes && (best == c->kept.end() || (*it)->n < (*best)->n)) best = it;
-        if (best != c->kept.end()) {
-            bufs.push_back(std::move(*best));
-            c->kept.erase(best);
-        } else {
-            auto b = std::make_unique<DevBuf>();
-            b->ensure(bytes);
-            bufs.push_back(std::move(b));
-        }
-        return bufs.back()->p;
+        if (best == c->kept.end()) return nullptr;
+        auto b = std::move(*best);
+        c->kept.erase(best);
+        return b;
     }
-    ~ScratchLease()
+    void give_back()
     {
-        if (std::uncaught_exceptions() > exceptions) cudaStreamSynchronize(s);
+        std::lock_guard<std::mutex> lk(g_kept_mu);
         size_t total = 0;
         for (auto& b : c->kept) total += b->n;
         for (auto& b : bufs) {
@@ -265,6 +259,28 @@ public:
             if (total + b->n > kScratchKeep) continue;
             total += b->n;
             c->kept.push_back(std::move(b));
+        }
+    }
+
+public:
+    ScratchLease(sun_ctx* c_, cudaStream_t s_) : c(c_), s(s_) {}
+    ScratchLease(const ScratchLease&) = delete;
+    void* get(size_t bytes)
+    {
+        auto b = take(bytes);
+        if (!b) {
+            b = std::make_unique<DevBuf>();
+            b->ensure(bytes);
+        }
+        bufs.push_back(std::move(b));
+        return bufs.back()->p;
+    }
+    ~ScratchLease()
+    {
+        if (std::uncaught_exceptions() > exceptions) cudaStreamSynchronize(s);
+        try {
+            give_back();
+        } catch (const std::bad_alloc&) {  // no room in the list: the rest is freed with bufs
         }
     }
 };
@@ -904,7 +920,7 @@ sun_status sun_init(const sun_config* cfg, sun_ctx** out)
         if (const char* t = getenv("SUN_B200_RESIDENT")) c->resident = atoi(t) ? 1 : 0;
         if (const char* t = getenv("SUN_B200_PDL")) c->pdl = atoi(t) ? 1 : 0;
         {
-            std::lock_guard<std::mutex> lk(g_ctxs_mu);
+            std::lock_guard<std::mutex> lk(g_kept_mu);
             g_ctxs.push_back(c.get());
         }
         *out = c.release();
@@ -915,7 +931,7 @@ sun_status sun_finalize(sun_ctx* c)
 {
     if (!c) return SUN_ERR_INVALID_ARG;
     {
-        std::lock_guard<std::mutex> lk(g_ctxs_mu);
+        std::lock_guard<std::mutex> lk(g_kept_mu);
         g_ctxs.erase(std::remove(g_ctxs.begin(), g_ctxs.end(), c), g_ctxs.end());
     }
     cudaStreamSynchronize(c->stream);
@@ -1137,6 +1153,15 @@ sun_status sun_ctx_hbm_budget(const sun_ctx* c, size_t* bytes)
     if (!c || !bytes) return SUN_ERR_INVALID_ARG;
     *bytes = c->hbm_budget;
     return SUN_OK;
+}
+
+sun_status sun_ctx_release_scratch(sun_ctx* c)
+{
+    if (!c) return SUN_ERR_INVALID_ARG;
+    return handle(c, [&] {
+        std::lock_guard<std::mutex> lk(g_kept_mu);
+        c->kept.clear();
+    });
 }
 
 sun_status sun_lattice_get_rng(sun_lattice* l, uint64_t* seed, uint32_t* hb, uint32_t* sw)
