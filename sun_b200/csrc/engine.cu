@@ -298,7 +298,10 @@ int work_of(const LatDev& L, int N, int kind)
         const int V3 = L.X[0] * L.X[1] * L.X[2], spw = 32 / poly_lanes(V3);
         return 32 * ((V3 + spw - 1) / spw);
     }
-    case WORK_LINKS8: return (4 * L.V + 7) / 8;
+    case WORK_REUNIT: {
+        const int n = reunit_links(L.V);
+        return (4 * L.V + n - 1) / n;
+    }
     default: return 4 * L.V;
     }
 }
@@ -520,8 +523,8 @@ int update_block(sun_ctx* c, Group& g, int mode, cudaStream_t s)
     return best;
 }
 
-// the scheduled reunitarization's view: few CTAs, most launches find it not due
-BatchView reunit_view(sun_ctx* c, Group& g, cudaStream_t s) { return g.view(WORK_LINKS8, c->blk_links, s); }
+// the scheduled reunitarization's view
+BatchView reunit_view(sun_ctx* c, Group& g, cudaStream_t s) { return g.view(WORK_REUNIT, c->blk_links, s); }
 
 // counters_later: the sweep's counter update is left to the launch after
 // it (the fused measurement of a sweep-and-measure graph); the
@@ -559,7 +562,9 @@ void group_sweep(sun_ctx* c, Group& g, int n_hb, int n_or, bool count_sweep, boo
     // end_sweep above also bumped the sweep counter when count_sweep; the
     // reunitarization kernel checks each lattice's own schedule on device
     if (reunit) {
-        OPS_CALL(g.N, reunit, g.fp64, g.layout, reunit_view(c, g, s), c->blk_links,
+        int loop = 0;
+        for (auto* l : g.lats) loop |= reunit_links(l->desc.V) > 1;
+        OPS_CALL(g.N, reunit, g.fp64, g.layout, reunit_view(c, g, s), loop, c->blk_links,
                  counters_later ? REUNIT_DUE_NEXT : REUNIT_DUE, s);
     }
 }
@@ -1482,7 +1487,7 @@ sun_status sun_reunitarize(sun_lattice* l, void* stream)
         cudaStream_t s = S(l->ctx, stream);
         Solo so(l);
         BatchView v = so.g.view(WORK_LINKS, l->ctx->blk_links, s);
-        OPS_CALL(l->p.ncolors, reunit, so.g.fp64, so.g.layout, v, l->ctx->blk_links, REUNIT_ALL, s);
+        OPS_CALL(l->p.ncolors, reunit, so.g.fp64, so.g.layout, v, 0, l->ctx->blk_links, REUNIT_ALL, s);
         ck(cudaStreamSynchronize(s), "reunitarize");
     });
 }

@@ -72,10 +72,23 @@ enum UpdateMode { MODE_HB = 0, MODE_HB_INJECTED = 1, MODE_OR = 2 };
 
 // Work per lattice a launch maps CTAs onto.
 // work items per lattice of a launch: half-sites, sites, spatial sites,
-// links (8 per thread: LINKS8), (site, plane) pairs of the plaquette (6 V), and
-// the lanes of the Polyakov loop's spatial sites (whole warps)
+// links, (site, plane) pairs of the plaquette (6 V), the lanes of the Polyakov
+// loop's spatial sites (whole warps), and the threads of a scheduled
+// reunitarization
 enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY = 5,
-                WORK_WILSON = 6, WORK_LINKS8 = 7 };
+                WORK_WILSON = 6, WORK_REUNIT = 7 };
+// links per thread of a scheduled reunitarization (k_reunit): one until the
+// launch has 16 CTAs of 256 threads per SM (148 SMs), then as many as leave 8 to
+// 16, at most eight.  Most launches find it not due and cost their CTAs' start
+// (within the noise of a 32^4 sweep), but a due launch lasts its longest thread,
+// so a smaller lattice keeps one.  One overrelaxation pass, reunitarized, us,
+// with one link / eight per thread: SU(2) FP32 8^4 23 / 27, SU(4) FP32 8^4 43 / 65,
+// SU(6) FP32 8^4 115 / 247; SU(3) FP64 24^4 with four / eight 398 / 405.
+__host__ __device__ inline int reunit_links(int V)
+{
+    const int n = 4 * V / (148 * 8 * 256);
+    return n < 1 ? 1 : (n > 8 ? 8 : n);
+}
 // lanes per spatial site of the Polyakov loop: 8 shorten the chain of a small
 // lattice; from kPolyFewV3 spatial sites up there are enough threads with 2
 constexpr int kPolyFewV3 = 8192;
@@ -169,9 +182,10 @@ template <int N> struct Ops {
     static int resident_capacity(int fp64, int layout, int rows);
     static cudaError_t cold(int fp64, int layout, const BatchView& bv, int block, cudaStream_t s);
     static cudaError_t hot(int fp64, int layout, const BatchView& bv, int block, cudaStream_t s);
-    // FP64 reunitarization of the lattices that `when` selects; the view may
-    // hold fewer threads than links
-    static cudaError_t reunit(int fp64, int layout, const BatchView& bv, int block, ReunitWhen when, cudaStream_t s);
+    // FP64 reunitarization of the lattices that `when` selects; loop: the view
+    // holds fewer threads than links
+    static cudaError_t reunit(int fp64, int layout, const BatchView& bv, int loop, int block, ReunitWhen when,
+                              cudaStream_t s);
     // per-CTA partials: plaquette 2 values, polyakov 2, unitarity 1 (max);
     // partial layout [block][value][sum, compensation]
     // plaquette and polyakov: with out non-null, the last CTA of each
