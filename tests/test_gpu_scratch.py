@@ -64,8 +64,8 @@ def test_kept_scratch_makes_room_for_a_lattice(busy):
                 time.sleep(0.3)
             big = gauge(b, N=3, dims=(24, 24, 24, 24), prec="f64")
             assert not busy or t.is_alive()
-            with pytest.raises(SunError) as e:  # nothing is kept any more
-                gauge(b, N=3, dims=(32, 32, 32, 32), prec="f64")
+            with pytest.raises(SunError) as e:  # 3 GB: more than any context keeps
+                gauge(b, N=3, dims=(48, 48, 48, 48), prec="f64")
             assert e.value.status == 3
         finally:
             if busy:
