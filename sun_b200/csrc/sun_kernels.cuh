@@ -1265,7 +1265,10 @@ template <int N> SUN_DEV void shfl_mat(Mat<N, double>& D, const Mat<N, double>& 
 // products plus log2 n joins instead of T products.  The 32 / n sites of a
 // warp are consecutive, each group's loads one segment of the image; FP32
 // links are loaded two products ahead.  32^4, cold: 29 us, 49 us with 8 lanes
-// per site and a product with the unit matrix first.
+// per site and a product with the unit matrix first.  SU(6), whose two FP64
+// matrices alone exceed the registers, loads each link where it is used: a
+// call on 4^4 FP32 22.7 us, 27.2 us with links loaded ahead (2.7 KB of spills
+// against 1.1 KB), 16^4 35.7 against 42.2 us.
 // Polyakov work item w of lattice L (thread w of k_polyakov's CTAs; all
 // lanes of the warp take part): the trace at the site of lane group k == 0,
 // links loaded through path P
@@ -1300,8 +1303,8 @@ SUN_DEV void polyakov_item(const LatDev& L, const Geom& g, int w, double& re, do
         // image index of U_3(x, t)
         int lex = lex_of(g, x), par = (x[0] + x[1] + x[2] + t0) & 1;
         auto index = [&] { return (L.evenodd ? (uint32_t)((lex >> 1) + par * g.halfV) : (uint32_t)lex) + mu3; };
-        constexpr int kAhead = sizeof(R) == 4 ? 2 : 1;
-        Mat<N, R> F[kAhead];
+        constexpr int kAhead = N > 4 ? 0 : (sizeof(R) == 4 ? 2 : 1);
+        Mat<N, R> F[kAhead ? kAhead : 1];
         auto next = [&](Mat<N, R>& to, int t) {
             if (t >= t1) return;
             IO::template load<P>(base, index(), stride, to);
@@ -1310,17 +1313,26 @@ SUN_DEV void polyakov_item(const LatDev& L, const Geom& g, int w, double& re, do
         };
         next(F[0], t0);
         mconvert(F[0], Pm);
-#pragma unroll
-        for (int i = 0; i < kAhead; ++i) next(F[i], t0 + 1 + i);
+        if constexpr (kAhead == 0) {
 #pragma unroll 1
-        for (int t = t0 + 1; t < t1; t += kAhead)
+            for (int t = t0 + 1; t < t1; ++t) {
+                next(F[0], t);
+                mconvert(F[0], A);
+                times(A);
+            }
+        } else {
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i)
-                if (t + i < t1) {
-                    mconvert(F[i], A);
-                    next(F[i], t + i + kAhead);
-                    times(A);
-                }
+            for (int i = 0; i < kAhead; ++i) next(F[i], t0 + 1 + i);
+#pragma unroll 1
+            for (int t = t0 + 1; t < t1; t += kAhead)
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i)
+                    if (t + i < t1) {
+                        mconvert(F[i], A);
+                        next(F[i], t + i + kAhead);
+                        times(A);
+                    }
+        }
     }
     // every lane of the warp takes part in the shuffles
 #pragma unroll 1
