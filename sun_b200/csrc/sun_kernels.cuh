@@ -260,9 +260,9 @@ template <class R> SUN_DEV cx<R> shfl_cx(cx<R> v, int src)
     return mkc<R>(__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src));
 }
 
-// Row-split k_update for small lattices of larger N.  The N lanes of a site
-// (32/N sites per warp) each multiply out one row of every staple product,
-// loading their row of its first factor and the whole of the others;
+// Row-split k_update for small lattices of N >= 3.  The N lanes of a site (32/N
+// sites per warp) each multiply out one row of every staple product, loading
+// their row of its first factor and the whole of the others;
 // the lanes then exchange their rows of the staple sum by warp shuffles, all
 // run the same update on the same inputs, and lane 0 stores the link.  Per
 // lane this holds far fewer live values than one thread per site (SU(6)
@@ -1213,10 +1213,10 @@ SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, d
             const double t = plaquette_plane<N, R, LAYOUT, P>(L, g, x, mu, nu);
             if (nu == 3) tp = t; else sp = t;
         }
-    } else if (w < g.V) {
+    } else if (P == LD_NC && w < g.V) {  // resident sweeps (LD_CG) have no such lattices
         int x[4];
         lex_coords(g, w, x);
-        if constexpr (kPlaquetteOwn<N> && P == LD_NC) {
+        if constexpr (kPlaquetteOwn<N>) {
             plaquette_site<N, R, LAYOUT>(L, g, x, own + threadIdx.x, blockDim.x, sp, tp);
         } else {
 #pragma unroll 1
@@ -1793,9 +1793,12 @@ SUN_DEV unsigned wait_count(const unsigned* count, unsigned target, int* status,
 // The waits of one update phase of a resident launch: `pre` the arrival
 // count at which the phase two back is complete (before any staple),
 // `dep_target` the count at which the previous phase is complete (before
-// the staple of its direction); 0: nothing to wait for.  Called by all lanes of a warp at
-// once: lane 0 polls (unless the CTA has seen the count already, *seen),
-// records the count seen, and the warp proceeds together.
+// the staple of its direction); 0: nothing to wait for.  Every lane of a
+// warp polls (one request for the warp, unless the CTA has seen the count
+// already, *seen), so the lanes leave the loop together.  With lane 0 polling
+// alone the warp stayed split behind the wait and ran its phases twice: SU(3)
+// FP64 8^4 456 us per sweep with 18 of 32 lanes active per instruction, 206 us
+// this way (SU(4) FP64 8^4 761 and 320 us).
 struct ResidentDep {
     const unsigned* count;
     int* status;
@@ -1804,15 +1807,13 @@ struct ResidentDep {
     unsigned* seen;
     SUN_DEV void wait_for(unsigned target) const
     {
-        if ((threadIdx.x & 31) == 0) {
-            if (*reinterpret_cast<volatile unsigned*>(seen) >= target) {
-                // another warp saw the count (its acquire fence, then the
-                // write of *seen); this fence makes the read an acquire
-                __threadfence_block();
-            } else {
-                const unsigned c = wait_count(count, target, status, wait_ns);
-                if (c) atomicMax(seen, c);
-            }
+        if (*reinterpret_cast<volatile unsigned*>(seen) >= target) {
+            // another warp saw the count (its acquire fence, then the
+            // write of *seen); this fence makes the read an acquire
+            __threadfence_block();
+        } else {
+            const unsigned c = wait_count(count, target, status, wait_ns);
+            if (c && (threadIdx.x & 31) == 0) atomicMax(seen, c);
         }
         __syncwarp();
     }
