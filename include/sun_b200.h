@@ -153,10 +153,13 @@ sun_status sun_sweep(sun_lattice *lat, int n_hb, int n_or, int n_sweeps, void *s
  * sun_sweep + sun_plaquette + sun_polyakov per sweep.  plaq[2i], plaq[2i+1]:
  * spatial and temporal plaquette after sweep i; poly[2i], poly[2i+1]:
  * Polyakov loop; host arrays of 2 n_sweeps doubles, either may be NULL.
- * One captured graph per sweep is replayed.  With SUN_B200_RESIDENT=1 a lattice
- * whose launch shapes allow it runs its sweeps in cooperative launches of up to
- * 256 sweeps whose grid barriers replace the launch boundaries, with the same
- * results (slower on B200); a barrier wait that runs out (one second) returns
+ * One captured graph per sweep is replayed, or the sweeps run in cooperative
+ * launches of up to 256 sweeps whose grid barriers replace the launch
+ * boundaries, with the same results: SU(3) FP32 full links of 9,216 and
+ * 12-parameter links of 6,145 up to 16,383 half-sites (SUN_B200_RESIDENT=0: never,
+ * 1: every class with N <= 4 below 2^15 sites, N = 4 below 2^17, whose launch
+ * shapes allow it, auto: the default; SUN_B200_RESIDENT_MAX_HALFV: a lower upper
+ * limit of the default).  A barrier wait that runs out (one second) returns
  * SUN_ERR_DEVICE_FLAG. */
 sun_status sun_sweep_measure(sun_lattice *lat, int n_hb, int n_or, int n_sweeps, double *plaq, double *poly,
                              void *stream);

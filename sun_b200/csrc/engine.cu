@@ -148,13 +148,18 @@ struct sun_ctx {
     int pdl = 1;
     long long rows_max_halfv = -1;  // SUN_B200_ROWS_MAX_HALFV (FP64: half of it); -1: rows_limit's own
     // sun_sweep_measure in cooperative launches (k_sweeps_resident) instead of
-    // a replayed graph: 1 whenever the lattice and launch shapes allow, 0 never
-    // (SUN_B200_RESIDENT; auto: never).  With the row-split kernel's phases
-    // overlapping, the graph is the faster one everywhere.  Measured on B200, 1
-    // HB + 4 OR with both observables per sweep, us per sweep resident / graph:
-    // SU(3) FP32 8^4 205 / 163 (12-parameter), 207 / 148 (full links), 14^4 276
-    // / 239; FP64 8^4 274 / 182.
-    int resident = 0;
+    // a replayed graph (SUN_B200_RESIDENT): 1 whenever the lattice and launch
+    // shapes allow, 0 never, -1 by size: SU(3) FP32 full and 12-parameter links
+    // from resident_min_halfv to resident_max_halfv half-sites.  Below, the graph
+    // of row-split phases is faster; from 2^15 sites up the plaquette's form
+    // (plaquette_site) has no resident counterpart.  Measured on B200, 1 HB + 4 OR with both observables
+    // per sweep, us per sweep resident / graph: full links 8^4 156 / 146-155, 10^4
+    // 182 / 166, 12^4 201 / 207, 12^3x14 209 / 219, 12^3x16 212 / 245;
+    // 12-parameter 8^4 172 / 167, 10^4 189 / 182, 8x12^3 192 / 208, 12^4 196 / 217,
+    // 12^3x16 204 / 225.  SOA8 416-442 / 399-445, SU(2) 120 / 98, SU(4) 8^4 241 /
+    // 214, SU(3) FP64 8^4 206 / 184: always the graph.
+    int resident = -1;
+    long long resident_max_halfv = 16384;  // SUN_B200_RESIDENT_MAX_HALFV
     unsigned long long barrier_wait_ns = 1000000000ull;  // one grid barrier wait at most
     int skip_arrive = -1;  // test hook (sun_debug_resident_barrier)
     DevBuf res_sync;       // barrier count, generation, status
@@ -922,7 +927,8 @@ sun_status sun_init(const sun_config* cfg, sun_ctx** out)
             else if (!strcmp(k, "tile")) c->upd_kernel = 3;
         }
         if (const char* t = getenv("SUN_B200_ROWS_MAX_HALFV")) c->rows_max_halfv = atoll(t);
-        if (const char* t = getenv("SUN_B200_RESIDENT")) c->resident = atoi(t) ? 1 : 0;
+        if (const char* t = getenv("SUN_B200_RESIDENT")) c->resident = !strcmp(t, "auto") ? -1 : (atoi(t) ? 1 : 0);
+        if (const char* t = getenv("SUN_B200_RESIDENT_MAX_HALFV")) c->resident_max_halfv = atoll(t);
         if (const char* t = getenv("SUN_B200_PDL")) c->pdl = atoi(t) ? 1 : 0;
         {
             std::lock_guard<std::mutex> lk(g_kept_mu);
@@ -1345,6 +1351,10 @@ static bool solo_measure_graph(sun_lattice* l, Group& g, int n_hb, int n_or, siz
 // sweeps per resident launch at most
 constexpr int kResidentChunk = 256;
 
+// half-sites of the smallest lattice that takes the resident path by default
+// (sun_ctx::resident): where its time crosses the graph's
+constexpr int resident_min_halfv(int layout) { return layout == SUN_SOA12 ? 6145 : 9216; }
+
 // sun_sweep_measure in cooperative launches (k_sweeps_resident), for a
 // lattice whose launched phases are latency-bound.  Returns false, having
 // launched nothing, when the lattice, the launch shapes or the stream do not
@@ -1355,6 +1365,9 @@ static bool resident_sweeps(sun_lattice* l, Group& g, int n_hb, int n_or, int n_
     sun_ctx* c = l->ctx;
     const LatDev& L = l->desc;
     if (c->resident == 0 || L.sweep_limit != 0u || c->blk_sites != 128 || g.N > 4) return false;
+    if (c->resident < 0 && (g.N != 3 || g.fp64 || g.layout == SUN_SOA8 || L.halfV > c->resident_max_halfv ||
+                            L.halfV < resident_min_halfv(g.layout)))
+        return false;
     if (L.V >= plane_split_max_v(g.N)) return false;  // their plaquette (plaquette_site) has no resident form
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
@@ -1362,16 +1375,25 @@ static bool resident_sweeps(sun_lattice* l, Group& g, int n_hb, int n_or, int n_
     // row-split kernel, CTAs of 128 threads, the same for both modes
     const int cfg_hb = n_hb > 0 ? update_block(c, g, MODE_HB, s) : 0;
     const int cfg_or = n_or > 0 ? update_block(c, g, MODE_OR, s) : 0;
-    const int cfg = n_hb > 0 ? cfg_hb : cfg_or;
+    int cfg = n_hb > 0 ? cfg_hb : cfg_or;
     if ((n_hb > 0 && n_or > 0 && cfg_hb != cfg_or) || (cfg != 128 && cfg != -128)) return false;
-    const int rows = cfg < 0;
-    int cap_ctas = 0;
-    switch (g.N) {
-    case 2: cap_ctas = Ops<2>::resident_capacity(g.fp64, g.layout, rows); break;
-    case 3: cap_ctas = Ops<3>::resident_capacity(g.fp64, g.layout, rows); break;
-    case 4: cap_ctas = Ops<4>::resident_capacity(g.fp64, g.layout, rows); break;
-    default: break;
+    const auto capacity = [&](int rows) {
+        switch (g.N) {
+        case 2: return Ops<2>::resident_capacity(g.fp64, g.layout, rows);
+        case 3: return Ops<3>::resident_capacity(g.fp64, g.layout, rows);
+        case 4: return Ops<4>::resident_capacity(g.fp64, g.layout, rows);
+        default: return 0;
+        }
+    };
+    int cap_ctas = capacity(cfg < 0);
+    // more row-split CTAs than SMs slow one another down (SU(3) FP32 full links,
+    // us per sweep, row-split / one thread per half-site: 8x12^3 (173 CTAs) 235 /
+    // 195, 12^4 (260) 423 / 201): one thread per half-site then, the same bits
+    if (cfg < 0 && upd_view(g, cfg, s).nblocks > std::min(cap_ctas / 2, 148)) {
+        cfg = 128;
+        cap_ctas = capacity(0);
     }
+    const int rows = cfg < 0;
     if (cap_ctas < 2) return false;
     BatchView upd = upd_view(g, cfg, s);
     BatchView vp = g.view(WORK_PLANES, 128, s), vl = g.view(WORK_POLY, 128, s);
