@@ -292,7 +292,8 @@ public:
 
 cudaStream_t S(sun_ctx* c, void* s) { return s ? reinterpret_cast<cudaStream_t>(s) : c->stream; }
 
-int work_of(const LatDev& L, int N, int kind)
+// work items of lattice L in a launch of `kind`; per: links per thread of WORK_REUNIT
+int work_of(const LatDev& L, int N, int kind, int per)
 {
     switch (kind) {
     case WORK_HALF: return L.halfV;
@@ -303,21 +304,18 @@ int work_of(const LatDev& L, int N, int kind)
         const int V3 = L.X[0] * L.X[1] * L.X[2], spw = 32 / poly_lanes(V3);
         return 32 * ((V3 + spw - 1) / spw);
     }
-    case WORK_REUNIT: {
-        const int n = reunit_links(L.V);
-        return (4 * L.V + n - 1) / n;
-    }
+    case WORK_REUNIT: return (4 * L.V + per - 1) / per;
     default: return 4 * L.V;
     }
 }
 
-int ctas_of(const LatDev& L, int N, int kind, int block)
+int ctas_of(const LatDev& L, int N, int kind, int block, int per)
 {
     if (kind == WORK_WILSON) {
         const int per = wilson_per_cta(L.V, block);
         return (wilson_items(L.V, block) + per - 1) / per;
     }
-    return (work_of(L, N, kind) + block - 1) / block;
+    return (work_of(L, N, kind, per) + block - 1) / block;
 }
 
 // Same-class lattices advanced by one launch per kernel.
@@ -344,6 +342,14 @@ struct Group {
         for (auto* l : lats)
             if (l->desc.V >= plane_split_max_v(N)) return 1;
         return 0;
+    }
+
+    // of a scheduled reunitarization
+    int links_per_thread() const
+    {
+        long long links = 0;
+        for (auto* l : lats) links += 4ll * l->desc.V;
+        return reunit_links(links);
     }
 
     void sync(cudaStream_t s)
@@ -374,7 +380,7 @@ struct Group {
         if (!e.valid) {
             std::vector<int> b(lats.size() + 1, 0);
             for (size_t i = 0; i < lats.size(); ++i)
-                b[i + 1] = b[i] + ctas_of(lats[i]->desc, N, kind, block);
+                b[i + 1] = b[i] + ctas_of(lats[i]->desc, N, kind, block, links_per_thread());
             if (!e.buf) e.buf = std::make_shared<DevBuf>();
             e.buf->ensure(sizeof(int) * b.size());
             ck(cudaMemcpyAsync(e.buf->p, b.data(), sizeof(int) * b.size(), cudaMemcpyHostToDevice, s), "begin upload");
@@ -567,9 +573,7 @@ void group_sweep(sun_ctx* c, Group& g, int n_hb, int n_or, bool count_sweep, boo
     // end_sweep above also bumped the sweep counter when count_sweep; the
     // reunitarization kernel checks each lattice's own schedule on device
     if (reunit) {
-        int loop = 0;
-        for (auto* l : g.lats) loop |= reunit_links(l->desc.V) > 1;
-        OPS_CALL(g.N, reunit, g.fp64, g.layout, reunit_view(c, g, s), loop, c->blk_links,
+        OPS_CALL(g.N, reunit, g.fp64, g.layout, reunit_view(c, g, s), g.links_per_thread() > 1, c->blk_links,
                  counters_later ? REUNIT_DUE_NEXT : REUNIT_DUE, s);
     }
 }

@@ -77,17 +77,18 @@ enum UpdateMode { MODE_HB = 0, MODE_HB_INJECTED = 1, MODE_OR = 2 };
 // reunitarization
 enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3, WORK_PLANES = 4, WORK_POLY = 5,
                 WORK_WILSON = 6, WORK_REUNIT = 7 };
-// links per thread of a scheduled reunitarization (k_reunit): one until the
-// launch has 16 CTAs of 256 threads per SM (148 SMs), then as many as leave 8 to
-// 16, at most eight.  Most launches find it not due and cost their CTAs' start
-// (within the noise of a 32^4 sweep), but a due launch lasts its longest thread,
-// so a smaller lattice keeps one.  One overrelaxation pass, reunitarized, us,
-// with one link / eight per thread: SU(2) FP32 8^4 23 / 27, SU(4) FP32 8^4 43 / 65,
-// SU(6) FP32 8^4 115 / 247; SU(3) FP64 24^4 with four / eight 398 / 405.
-__host__ __device__ inline int reunit_links(int V)
+// links per thread of a scheduled reunitarization (k_reunit) whose lattices have
+// `links` links in all: one until the launch has 16 CTAs of 256 threads per SM
+// (148 SMs), then as many as leave 8 to 16, at most eight.  Most launches find it
+// not due and cost their CTAs' start (within the noise of a 32^4 sweep), but a due
+// launch lasts its longest thread, so a small lattice keeps one.  One
+// overrelaxation pass, reunitarized, us, with one link / eight per thread: SU(2)
+// FP32 8^4 23 / 27, SU(4) FP32 8^4 43 / 65, SU(6) FP32 8^4 115 / 247; SU(3) FP64 24^4
+// with four / eight 398 / 405.
+inline int reunit_links(long long links)
 {
-    const int n = 4 * V / (148 * 8 * 256);
-    return n < 1 ? 1 : (n > 8 ? 8 : n);
+    const long long n = links / (148 * 8 * 256);
+    return n < 1 ? 1 : (n > 8 ? 8 : (int)n);
 }
 // lanes per spatial site of the Polyakov loop: 8 shorten the chain of a small
 // lattice; from kPolyFewV3 spatial sites up there are enough threads with 2
