@@ -153,11 +153,11 @@ struct sun_ctx {
     // from resident_min_halfv to resident_max_halfv half-sites.  Below, the graph
     // of row-split phases is faster; from 2^15 sites up the plaquette's form
     // (plaquette_site) has no resident counterpart.  Measured on B200, 1 HB + 4 OR with both observables
-    // per sweep, us per sweep resident / graph: full links 8^4 156 / 146-155, 10^4
-    // 182 / 166, 12^4 201 / 207, 12^3x14 209 / 219, 12^3x16 212 / 245;
-    // 12-parameter 8^4 172 / 167, 10^4 189 / 182, 8x12^3 192 / 208, 12^4 196 / 217,
-    // 12^3x16 204 / 225.  SOA8 416-442 / 399-445, SU(2) 120 / 98, SU(4) 8^4 241 /
-    // 214, SU(3) FP64 8^4 206 / 184: always the graph.
+    // per sweep, us per sweep resident / graph: full links 8^4 156 / 149-156, 10^4
+    // 183 / 164, 8x12^3 188 / 186, 12^4 200 / 208, 12^3x16 210 / 236-244;
+    // 12-parameter 8^4 176 / 171, 10^4 190 / 178-183, 8x12^3 187 / 204, 12^4 195 /
+    // 216, 12^3x16 205 / 225.  SOA8 8^4 425 / 400, SU(2) 8^4 117 / 106, SU(4) 8^4 240
+    // / 204-210, SU(3) FP64 8^4 206 / 191: always the graph.
     int resident = -1;
     long long resident_max_halfv = 16384;  // SUN_B200_RESIDENT_MAX_HALFV
     unsigned long long barrier_wait_ns = 1000000000ull;  // one grid barrier wait at most
@@ -631,7 +631,8 @@ void group_plaquette(sun_ctx* c, Group& g, double* out, cudaStream_t s)
 {
     double* r = group_reduce_fused(g, WORK_PLANES, c->blk_sites, 2, s,
                                    [&](const BatchView& v, double* part, double* out, unsigned* cnt) {
-                                       OPS_CALL(g.N, plaquette, g.fp64, g.layout, v, g.large(), c->blk_sites, part, out, cnt, nullptr, s);
+                                       OPS_CALL(g.N, plaquette, g.fp64, g.layout, v, g.large(), c->blk_sites, part,
+                                                out, cnt, nullptr, s);
                                    });
     for (size_t i = 0; i < g.lats.size(); ++i) {
         const LatDev& L = g.lats[i]->desc;
@@ -1328,8 +1329,8 @@ static bool solo_measure_graph(sun_lattice* l, Group& g, int n_hb, int n_or, siz
         group_sweep(c, g, n_hb, n_or, true, re, cs, fused);
         if (fused) {
             unsigned* mc = reinterpret_cast<unsigned*>(l->meas_cnt.p);
-            OPS_CALL(g.N, plaq_poly, g.fp64, g.layout, vp, g.large(), vl, part, part + 4 * (size_t)vp.nblocks, out_p, out_l, mc,
-                     mc + 1, slot, mc + 2, n_hb, cs);
+            OPS_CALL(g.N, plaq_poly, g.fp64, g.layout, vp, g.large(), vl, part, part + 4 * (size_t)vp.nblocks, out_p,
+                     out_l, mc, mc + 1, slot, mc + 2, n_hb, cs);
         } else {
             OPS_CALL(g.N, plaquette, g.fp64, g.layout, vp, g.large(), c->blk_sites, part, out_p, cnt, slot, cs);
             OPS_CALL(g.N, polyakov, g.fp64, g.layout, vl, c->blk_sites, part, out_l, cnt, slot, cs);
@@ -1604,7 +1605,8 @@ void check_dirmask(int dirmask)
 // from 2^25 sites in FP64, 2^26 in FP32), a plain copy per element and run
 void copy_directions(sun_lattice* l, void* dst, const void* src, int dirmask, cudaStream_t s)
 {
-    const size_t csz = l->p.precision == SUN_F64 ? 16 : 8, row = csz * (size_t)l->desc.V;  // one direction of one element
+    const size_t csz = l->p.precision == SUN_F64 ? 16 : 8;
+    const size_t row = csz * (size_t)l->desc.V;  // one direction of one element
     const int elems = elems_of(l->p.ncolors, l->p.layout);
     int max_pitch = 0;
     ck(cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, l->ctx->device), "max pitch");
@@ -1624,7 +1626,8 @@ void copy_directions(sun_lattice* l, void* dst, const void* src, int dirmask, cu
 }
 
 // step(group, view, image of the selected directions, image to write)
-template <class F> void smear_steps(sun_lattice* l, int steps, int dirmask, ScratchLease& scratch, cudaStream_t s, F step)
+template <class F>
+void smear_steps(sun_lattice* l, int steps, int dirmask, ScratchLease& scratch, cudaStream_t s, F step)
 {
     if (steps <= 0) return;
     void* img[2] = {scratch.get(l->bytes), l->links.p};

@@ -974,8 +974,8 @@ SUN_DEV void block_sum2(double v0, double v1, double* out, DD* sh)
 }
 // The sums of CTA partials b0 .. b1 - 1 (two values each), by a whole CTA:
 // thread-strided compensated sums, then cta_sum2; thread v writes value v to
-// dst[v].  (One warp
-// walking the partials of a 32^4 plaquette, 8,192 CTAs, took 80 us.)
+// dst[v].  (One warp walking the partials of a 32^4 plaquette, 8,192 CTAs, took
+// 80 us.)
 SUN_DEV void finalize_partials(const double* partials, int b0, int b1, double* dst, DD* sh)
 {
     DD d[2] = {{0.0, 0.0}, {0.0, 0.0}};
@@ -1231,8 +1231,8 @@ SUN_DEV void plaquette_item(const LatDev& L, const Geom& g, int w, double& sp, d
 }
 
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128, N <= 3 ? 3 : 1) k_plaquette(BatchView bv, double* partials, double* out, unsigned* counters,
-                                                    const unsigned* slot)
+__global__ void __launch_bounds__(128, N <= 3 ? 3 : 1)
+    k_plaquette(BatchView bv, double* partials, double* out, unsigned* counters, const unsigned* slot)
 {
     extern __shared__ __align__(16) unsigned char plaquette_raw[];
     __shared__ DD sh[32];
@@ -1350,8 +1350,8 @@ SUN_DEV void polyakov_item(const LatDev& L, const Geom& g, int w, double& re, do
 }
 
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128, N <= 3 ? 4 : 1) k_polyakov(BatchView bv, double* partials, double* out, unsigned* counters,
-                                                   const unsigned* slot)
+__global__ void __launch_bounds__(128, N <= 3 ? 4 : 1)
+    k_polyakov(BatchView bv, double* partials, double* out, unsigned* counters, const unsigned* slot)
 {
     __shared__ DD sh[32];
     const int b = blockIdx.x;
@@ -1373,9 +1373,9 @@ __global__ void __launch_bounds__(128, N <= 3 ? 4 : 1) k_polyakov(BatchView bv, 
 // advances *slot for the next replay and, with end_n_hb >= 0, ends the sweep
 // (the counters, which the measurements do not read).
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128, N <= 3 ? 3 : 1) k_plaq_poly(BatchView vp, BatchView vl, double* part_p, double* part_l,
-                                                    double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
-                                                    unsigned* slot, unsigned* joint, int end_n_hb)
+__global__ void __launch_bounds__(128, N <= 3 ? 3 : 1)
+    k_plaq_poly(BatchView vp, BatchView vl, double* part_p, double* part_l, double* out_p, double* out_l,
+                unsigned* cnt_p, unsigned* cnt_l, unsigned* slot, unsigned* joint, int end_n_hb)
 {
     extern __shared__ __align__(16) unsigned char plaquette_raw[];
     __shared__ DD sh[32];
@@ -1599,7 +1599,9 @@ __global__ void __launch_bounds__(128, WilsonOccupancy<N>::min_blocks) k_wilson(
 // Sums of a lattice's CTAs, one warp per (lattice, slot); out in the order
 // W[t + r (T + 1)] (Re, Im), unnormalised: the entries a launch does not sum
 // are 3 N V (r = t = 0) and the zero imaginary parts of r t = 0.
-template <int N> __global__ void __launch_bounds__(32) k_wilson_finalize(BatchView bv, int RR, int TT, const double2* partials, double* out)
+template <int N>
+__global__ void __launch_bounds__(32) k_wilson_finalize(BatchView bv, int RR, int TT, const double2* partials,
+                                                         double* out)
 {
     const int l = blockIdx.x, i = blockIdx.y, lane = threadIdx.x;
     double* o = out + (size_t)l * 2 * (RR + 1) * (TT + 1);
@@ -2174,9 +2176,9 @@ cudaError_t Ops<N>::plaquette(int fp64, int layout, const BatchView& bv, int lar
 {
     const int smem = large ? plaquette_smem<N>(block) : 0;
     cudaError_t e = cudaSuccess;
-#define CALL(R_, L_)                                                                                        \
-    if ((e = smem ? allow_smem<k_plaquette<N, R_, L_>>(plaquette_smem<N>(128)) : cudaSuccess) == cudaSuccess)                               \
-        k_plaquette<N, R_, L_><<<bv.nblocks, block, smem, s>>>(bv, partials, out, counters, slot)
+#define CALL(R_, L_)                                                           \
+    if (smem) e = allow_smem<k_plaquette<N, R_, L_>>(plaquette_smem<N>(128));  \
+    if (e == cudaSuccess) k_plaquette<N, R_, L_><<<bv.nblocks, block, smem, s>>>(bv, partials, out, counters, slot)
     SUN_DISPATCH(fp64, layout, CALL);
 #undef CALL
     return e != cudaSuccess ? e : cudaGetLastError();
@@ -2200,7 +2202,8 @@ cudaError_t Ops<N>::plaq_poly(int fp64, int layout, const BatchView& vp, int lar
     const int smem = large ? plaquette_smem<N>(128) : 0;
     cudaError_t e = cudaSuccess;
 #define CALL(R_, L_)                                                                                            \
-    if ((e = smem ? allow_smem<k_plaq_poly<N, R_, L_>>(plaquette_smem<N>(128)) : cudaSuccess) == cudaSuccess)                                   \
+    if (smem) e = allow_smem<k_plaq_poly<N, R_, L_>>(smem);                                                     \
+    if (e == cudaSuccess)                                                                                       \
         k_plaq_poly<N, R_, L_><<<vp.nblocks + vl.nblocks, 128, smem, s>>>(vp, vl, part_p, part_l, out_p, out_l, \
                                                                           cnt_p, cnt_l, slot, joint, end_n_hb)
     SUN_DISPATCH(fp64, layout, CALL);

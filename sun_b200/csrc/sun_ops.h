@@ -98,7 +98,10 @@ __host__ __device__ inline int poly_lanes(int V3) { return V3 < kPolyFewV3 ? 8 :
 // spatial direction), item i = 3 tile + mu, and a CTA takes wilson_per_cta
 // consecutive ones.  kWilsonCtas: the CTAs of one lattice at most -- 3 per SM,
 // what the shared memory of N = 3, T = 4 lets reside, so one lattice's items
-// are spread evenly over one wave.  Both depend on the lattice and the loop
+// are spread evenly over one wave.  It is tuned for that case only: of N = 2 four
+// CTAs per SM could reside, of N = 4 with T >= 5 five one-warp ones, of N = 6 with
+// T >= 5 one or two (calls, R = T = 4 / 8: SU(2) 24^3x48 0.72 / 2.3 ms, SU(4) 24^4
+// 1.9 / 10.8 ms, SU(6) 16^4 3.6 / 22 ms).  Both depend on the lattice and the loop
 // extents alone, so the sums have the same bits alone and in a batch.
 constexpr int kWilsonCtas = 444;
 __host__ __device__ inline int wilson_items(int V, int block) { return 3 * ((V + block - 1) / block); }
@@ -203,8 +206,8 @@ template <int N> struct Ops {
     // end_n_hb >= 0: the same launch ends the sweep (advance_counters with
     // n_hb = end_n_hb, one sweep) after the measurements
     static cudaError_t plaq_poly(int fp64, int layout, const BatchView& vp, int large, const BatchView& vl,
-                                 double* part_p, double* part_l, double* out_p, double* out_l, unsigned* cnt_p, unsigned* cnt_l,
-                                 unsigned* slot, unsigned* joint, int end_n_hb, cudaStream_t s);
+                                 double* part_p, double* part_l, double* out_p, double* out_l, unsigned* cnt_p,
+                                 unsigned* cnt_l, unsigned* slot, unsigned* joint, int end_n_hb, cudaStream_t s);
     // Wilson loops: bv a WORK_WILSON view for wilson_block(N, R, T); partials
     // hold wilson_slots(R, T) (sum, compensation) pairs per CTA, out
     // 2 (R + 1)(T + 1) sums per lattice (host-mapped memory allowed)

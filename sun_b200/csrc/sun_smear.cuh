@@ -5,8 +5,8 @@
 // Every kernel of a smearing step reads the unchanged field and writes `dst`:
 // the smeared directions (dirmask) from `src`, the others from the lattice's
 // own image (src and dst are distinct images of its layout, order and
-// precision; one of them may be that image), one thread per site and one grid row (blockIdx.y) per smeared direction or intermediate
-// link, so a smearing step is one launch (three for HYP) whatever the
+// precision; one of them may be that image), one thread per site and one grid
+// row (blockIdx.y) per smeared direction or intermediate link, so a smearing step is one launch (three for HYP) whatever the
 // directions.  The reference allows only normal-order SOA arrays here
 // (src/smear/ape.cu:194-197); these kernels take any storage order and layout.
 #pragma once
@@ -215,8 +215,8 @@ template <class R> SUN_DEV void exp_iq3(const Mat<3, R>& Q, Mat<3, R>& E)
 // 24^4, copy and three steps: 1.32 ms with a square root and a division per
 // subgroup, 1.18 ms with rsqrt; 1.24 ms capped at 128 registers (four CTAs, spills).
 template <int N, class R, int LAYOUT>
-__global__ void __launch_bounds__(128, N == 3 && sizeof(R) == 8 ? 3 : 1) k_ape(BatchView bv, const void* src, void* dst, int dirmask, R w, int nhits,
-                                             R tol)
+__global__ void __launch_bounds__(128, N == 3 && sizeof(R) == 8 ? 3 : 1)
+    k_ape(BatchView bv, const void* src, void* dst, int dirmask, R w, int nhits, R tol)
 {
     const int b = blockIdx.x;
     const int l = find_lat(bv, b);
