@@ -80,11 +80,11 @@ enum WorkKind { WORK_HALF = 0, WORK_SITES = 1, WORK_SPATIAL = 2, WORK_LINKS = 3,
 // links per thread of a scheduled reunitarization (k_reunit) whose lattices have
 // `links` links in all: one until the launch has 16 CTAs of 256 threads per SM
 // (148 SMs), then as many as leave 8 to 16, at most eight.  Most launches find it
-// not due and cost their CTAs' start (within the noise of a 32^4 sweep), but a due
-// launch lasts its longest thread, so a small lattice keeps one.  One
-// overrelaxation pass, reunitarized, us, with one link / eight per thread: SU(2)
-// FP32 8^4 23 / 27, SU(4) FP32 8^4 43 / 65, SU(6) FP32 8^4 115 / 247; SU(3) FP64 24^4
-// with four / eight 398 / 405.
+// not due and cost their CTAs' start (SU(3) 32^4, every tenth sweep due: 19 us per
+// sweep with one link per thread, 9 with eight), but a due launch lasts its longest
+// thread, so a small lattice keeps one.  One overrelaxation pass, reunitarized, us,
+// with one link / eight per thread: SU(2) FP32 8^4 23 / 27, SU(4) FP32 8^4 43 / 65,
+// SU(6) FP32 8^4 115 / 247; SU(3) FP64 24^4 with four / eight 398 / 405.
 inline int reunit_links(long long links)
 {
     const long long n = links / (148 * 8 * 256);
